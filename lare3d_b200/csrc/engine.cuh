@@ -406,6 +406,37 @@ template <class R> inline void end_of_step_bcs(Run<R>& r) {
   ghost_flush(r, b);
 }
 
+// Blocks of kernel K (threads a block, dynamic shared memory smem) that fit
+// on the GPU at once.
+template <auto K>
+inline int resident_blocks(int threads, size_t smem = 0) {
+  static const int n = [&] {
+    int b = 0, dev = 0, sms = 148;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, K, threads, smem);
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return (b > 0 ? b : 1) * sms;
+  }();
+  return n;
+}
+// Points of a marched axis of length len that one block of a marching kernel
+// walks, for a launch of `tiles` blocks across it, `resident` of which fit on
+// the GPU at once.  A chunk loads its stencil again, so longer is cheaper: cap
+// where that still makes two full waves, else as long as one wave allows (a
+// second, partial one would cost as much as the first), down to 4 on small
+// grids, where the march's latency is the kernel's time.  With fixed chunks of
+// 16 and 32 a 64^3 grid left most SMs idle: the march of eta_calc took 52 us
+// on 96 x 80 x 121 with 8 % of the resident blocks launched.
+inline int march_chunk(int len, int tiles, int cap, int resident) {
+  int n = (len + cap - 1) / cap;
+  if ((long long)tiles * n < 2LL * resident) {
+    n = resident / tiles;
+    if (n < 1) n = 1;
+    if (n > (len + 3) / 4) n = (len + 3) / 4;
+  }
+  return (len + n - 1) / n;
+}
+
 // Full-array elementwise helpers (Fortran whole-array statements).
 template <class R, class Fn>
 inline void whole(Run<R>& r, Fn fn) {

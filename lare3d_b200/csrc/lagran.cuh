@@ -63,7 +63,7 @@ __device__ __forceinline__ void vertex_current(const R* bx, const R* by, const R
 // (bx(c+Y+Z)-bx(c+Z))/dyc, are the next vertex's jz1 terms; a step loads
 // 8 values and divides 10 times instead of 12 and 12.  Same expressions,
 // same operands, same results bit for bit.
-constexpr int kEtaZ = 32;
+constexpr int kEtaZ = 32;  // largest chunk of z (march_chunk)
 
 template <class R>
 struct EtaArgs {
@@ -79,6 +79,7 @@ struct EtaArgs {
   A1<R> dxc, dyc, dzc;
   R jmax, eb, e0;
   int nx, ny, nz, sx, sxy;
+  int chunk;
   bool rkstep;
 };
 
@@ -101,8 +102,8 @@ __global__ void __launch_bounds__(128) k_eta_march(EtaArgs<R> g) {
   const int ix = -1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int iy = -1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (ix > g.nx + 1 || iy > g.ny + 1) return;
-  const int z0 = -1 + (int)blockIdx.z * kEtaZ;
-  const int z1 = min(z0 + kEtaZ - 1, g.nz + 1);
+  const int z0 = -1 + (int)blockIdx.z * g.chunk;
+  const int z1 = min(z0 + g.chunk - 1, g.nz + 1);
   const int sx = g.sx, sxy = g.sxy;
   const R dxc = g.dxc(ix), dyc = g.dyc(iy);
   const R vxc = dv_of(dxc), vyc = dv_of(dyc);  // divisors in the variant's form
@@ -209,7 +210,9 @@ void eta_and_rkstep(Run<R>& run, bool with_rkstep) {
   ga.sx = sx;
   ga.sxy = sxy;
   ga.rkstep = with_rkstep;
-  dim3 grd((nx + 3 + 31) / 32, (ny + 3 + 3) / 4, (nz + 3 + kEtaZ - 1) / kEtaZ);
+  dim3 grd((nx + 3 + 31) / 32, (ny + 3 + 3) / 4, 1);
+  ga.chunk = march_chunk(nz + 3, grd.x * grd.y, kEtaZ, resident_blocks<k_eta_march<R, false>>(128));
+  grd.z = (nz + 3 + ga.chunk - 1) / ga.chunk;
   const int k = run.prof_begin("eta_and_rkstep", 0, with_rkstep ? 8 : 4, (double)(nx + 3) * (ny + 3) * (nz + 3));
   if (with_rkstep && run.cowling)
     k_eta_march<R, true><<<grd, dim3(32, 4, 1), 0, run.s>>>(ga);
@@ -452,7 +455,9 @@ void prologue_and_shock_viscosity(Run<R>& run) {
     l4.sx = sx;
     l4.sxy = sxy;
     const dim3 blk(kL4X, kL4Y, 1);
-    const dim3 grd((nx + 2 + kL4X - 1) / kL4X, (ny + 2 + kL4Y - 1) / kL4Y, (nz + 2 + kL4Z - 1) / kL4Z);
+    dim3 grd((nx + 2 + kL4X - 1) / kL4X, (ny + 2 + kL4Y - 1) / kL4Y, 1);
+    l4.chunk = march_chunk(nz + 2, grd.x * grd.y, kL4Z, resident_blocks<k_lp4_tile<R>>(kL4X * kL4Y, lp4_smem_bytes<R>()));
+    grd.z = (nz + 2 + l4.chunk - 1) / l4.chunk;
     const int k = run.prof_begin("shock_viscosity_lp4_tile", 0, 13, (double)(nx + 2) * (ny + 2) * (nz + 2));
     k_lp4_tile<R><<<grd, blk, lp4_smem_bytes<R>(), run.s>>>(l4);
     run.prof_end(k);
@@ -619,7 +624,7 @@ void predictor_remap(Run<R>& run, int step) {
 // corner values (a register-window march needed 130 registers and ran
 // 0.59-0.64 ms against 0.55 ms at 256^3 in FP64, 0.33 against 0.30 ms in
 // FP32).  Same expressions, same operands, same results bit for bit.
-constexpr int kShockZ = 32;
+constexpr int kShockZ = 32;  // largest chunk of z (march_chunk)
 
 template <class R>
 struct ShockArgs {
@@ -632,6 +637,7 @@ struct ShockArgs {
   R* nv[3];
   A1<R> dxb, dyb, dzb;
   int nx, ny, nz, sx, sxy;
+  int chunk;
 };
 
 constexpr int kShX = 32, kShY = 8;
@@ -643,8 +649,8 @@ __global__ void __launch_bounds__(kShX * kShY, sizeof(R) == 8 ? 2 : 4) k_shock_t
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kShX + tx;
   const int ix0 = blockIdx.x * kShX, iy0 = blockIdx.y * kShY;
   const int ix = ix0 + tx, iy = iy0 + ty;
-  const int z0 = (int)blockIdx.z * kShockZ;
-  const int z1 = min(z0 + kShockZ - 1, g.nz + 1);
+  const int z0 = (int)blockIdx.z * g.chunk;
+  const int z1 = min(z0 + g.chunk - 1, g.nz + 1);
   const int sx = g.sx, sxy = g.sxy;
   const bool cell = ix <= g.nx + 1 && iy <= g.ny + 1;
   // the plane elements this thread loads (vertex x in ix0-1..ix0+31, y in
@@ -868,7 +874,9 @@ void predictor_corrector_step(Run<R>& run) {
     ga.sx = sx;
     ga.sxy = sxy;
     dim3 blk(kShX, kShY, 1);
-    dim3 grd((nx + 2 + kShX - 1) / kShX, (ny + 2 + kShY - 1) / kShY, (nz + 2 + kShockZ - 1) / kShockZ);
+    dim3 grd((nx + 2 + kShX - 1) / kShX, (ny + 2 + kShY - 1) / kShY, 1);
+    ga.chunk = march_chunk(nz + 2, grd.x * grd.y, kShockZ, resident_blocks<k_shock_tile<R>>(kShX * kShY));
+    grd.z = (nz + 2 + ga.chunk - 1) / ga.chunk;
     const int k = run.prof_begin("shock_heating", 0, 14, (double)(nx + 2) * (ny + 2) * (nz + 2));
     k_shock_tile<R><<<grd, blk, 0, run.s>>>(ga);
     run.prof_end(k);

@@ -6,7 +6,7 @@
 // y-1..y, z-1..z), the edge viscosities alpha1..3 of the cell and of its
 // neighbours, and per vertex (0:n) the velocity at the vertex and its six
 // neighbours.  A CTA of 32 x 8 threads owns a 32 x 8 column and walks a
-// 16-plane chunk of z with the planes of vx, vy, vz, alpha1, alpha2 and
+// chunk of z (16 planes at 256^3) with the planes of vx, vy, vz, alpha1, alpha2 and
 // alpha3 (a one-point x/y halo on each side) in a ring of four
 // shared-memory slots; plane z+2 is copied into the fourth by cp.async
 // while plane z is computed, so no register holds a plane in flight.  Every
@@ -21,7 +21,7 @@
 
 LARE_BEGIN
 
-constexpr int kL4X = 32, kL4Y = 8, kL4Z = 16;
+constexpr int kL4X = 32, kL4Y = 8, kL4Z = 16;  // tile, largest chunk of z (march_chunk)
 constexpr int kL4W = kL4X + 2;           // plane row with a one-vertex halo each side
 constexpr int kL4P = kL4W * (kL4Y + 2);  // plane size
 
@@ -42,6 +42,7 @@ struct LP4Args {
   R* fz;
   A1<R> dxb, dyb, dzb, dxc, dyc, dzc;
   int nx, ny, nz, sx, sxy;
+  int chunk;
 };
 
 // Dynamic shared memory of k_lp4_tile: four slots of six planes.
@@ -57,8 +58,8 @@ __global__ void __launch_bounds__(kL4X * kL4Y, sizeof(R) == 8 ? 3 : 4) k_lp4_til
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kL4X + tx;
   const int ix0 = blockIdx.x * kL4X, iy0 = blockIdx.y * kL4Y;
   const int ix = ix0 + tx, iy = iy0 + ty;
-  const int iz0 = blockIdx.z * kL4Z;
-  const int iz1 = min(iz0 + kL4Z - 1, g.nz + 1);
+  const int iz0 = blockIdx.z * g.chunk;
+  const int iz1 = min(iz0 + g.chunk - 1, g.nz + 1);
   const int sx = g.sx, sxy = g.sxy;
   const bool cell = ix <= g.nx + 1 && iy <= g.ny + 1;
   const bool vert = ix <= g.nx && iy <= g.ny;

@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(128) k_bflux_march1(BfArgs<R> a) {
 // carried from the previous step instead of reloaded, and the z face below a
 // cell is the previous step's z face above it: 12 to 15 loads per cell
 // instead of 28, the same expressions, the same results bit for bit.
-constexpr int kGeomZ = 16;
+constexpr int kGeomZ = 16;  // largest chunk of z (march_chunk)
 
 template <class R>
 struct GeomArgs {
@@ -412,6 +412,7 @@ struct GeomArgs {
   R pass_t1, pass_t2;
   const double* sc;
   int dt_slot, nx, ny, nz, sx, sxy;
+  int chunk;
   bool write_cv2;
 };
 
@@ -431,8 +432,8 @@ __global__ void __launch_bounds__(128) k_geom_march(GeomArgs<R> g) {
   const int ix = -1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int iy = -1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (ix > g.nx + 2 || iy > g.ny + 2) return;
-  const int z0 = -1 + (int)blockIdx.z * kGeomZ;
-  const int z1 = min(z0 + kGeomZ - 1, g.nz + 2);
+  const int z0 = -1 + (int)blockIdx.z * g.chunk;
+  const int z1 = min(z0 + g.chunk - 1, g.nz + 2);
   const int sx = g.sx, sxy = g.sxy;
   const int nn[3] = {g.nx, g.ny, g.nz};
   const R q4 = R(0.25);
@@ -688,7 +689,7 @@ __global__ void __launch_bounds__(128) k_vert_march(VertArgs<R> g) {
 // bounds) is the measured best per precision.  Every flux and update is the
 // reference's expression over the same operands, so the results are
 // identical bit for bit.
-constexpr int kMomA = 32;
+constexpr int kMomA = 32;  // largest chunk (march_chunk)
 
 template <class R>
 struct MomArgs {
@@ -706,6 +707,7 @@ struct MomArgs {
   A1<R> dct1, dct2;
   const double* sc;
   int dt_slot, nx, ny, nz, na, n3, sx, sxy, SA, S3;
+  int chunk;
 };
 
 // the three momentum fluxes through a face (K8's body) from its stencil
@@ -823,8 +825,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 4 : 8) k_mom_march(MomAr
   const int t0 = (int)(blockIdx.x * blockDim.x + threadIdx.x);  // x, 0..nx
   const int t1 = (int)(blockIdx.y * blockDim.y + threadIdx.y);  // the third axis, 0..n3
   if (t0 > g.nx || t1 > g.n3) return;
-  const int ia0 = (int)blockIdx.z * kMomA;
-  const int ia1 = min(ia0 + kMomA - 1, g.na);
+  const int ia0 = (int)blockIdx.z * g.chunk;
+  const int ia1 = min(ia0 + g.chunk - 1, g.na);
   const R dt = (R)g.sc[g.dt_slot];
   const int SA = g.SA;
   const R area = g.dct1(t0) * g.dct2(t1);
@@ -1013,7 +1015,7 @@ __global__ void __launch_bounds__(128) k_bupdate(BUpdArgs<R> g) {
 // energy goes to a second buffer (swapped in after the launch) because the
 // limiter of the next chunk still reads the old values.  The same
 // expressions over the same operands as the three point kernels.
-constexpr int kMEChunk = 16;
+constexpr int kMEChunk = 16;  // largest chunk (march_chunk)
 
 template <class R>
 struct MEArgs {
@@ -1032,6 +1034,7 @@ struct MEArgs {
   int dt_slot;
   int SA, S1, S2, SY;  // strides along A, T1 (= x), T2, and the thread grid's second axis (= T2)
   int na, nt1, nt2;
+  int chunk;
   bool per;
 };
 
@@ -1041,8 +1044,8 @@ __global__ void __launch_bounds__(128) k_mass_energy_march(MEArgs<R> a) {
   const int t = (int)(blockIdx.y * blockDim.y + threadIdx.y) - 1;  // T2, -1..nt2+2
   if (x > a.nt1 + 2 || t > a.nt2 + 2) return;
   const int na = a.na, SA = a.SA, S1 = a.S1, S2 = a.S2;
-  const int ia0 = -1 + (int)blockIdx.z * kMEChunk;
-  const int ia1 = min(ia0 + kMEChunk - 1, na + 2);
+  const int ia0 = -1 + (int)blockIdx.z * a.chunk;
+  const int ia1 = min(ia0 + a.chunk - 1, na + 2);
   const bool inside_t = x >= 0 && x <= a.nt1 + 1 && t >= 0 && t <= a.nt2 + 1;  // dm's transverse range
   const bool line0 = x <= a.nt1 && t <= a.nt2 && x >= 0 && t >= 0;          // the energy flux's
   const bool line1 = line0 && x >= 1 && t >= 1;                              // the updates'
@@ -1331,7 +1334,9 @@ void remap_sweep(Run<R>& run, bool predictor, int dt_slot, int pass[3], int bmod
     ga.sxy = sxy;
     ga.write_cv2 = write_cv2;
     dim3 blk(32, 4, 1);
-    dim3 grd((nx + 4 + 31) / 32, (ny + 4 + 3) / 4, (nz + 4 + kGeomZ - 1) / kGeomZ);
+    dim3 grd((nx + 4 + 31) / 32, (ny + 4 + 3) / 4, 1);
+    ga.chunk = march_chunk(nz + 4, grd.x * grd.y, kGeomZ, resident_blocks<k_geom_march<A, R>>(128));
+    grd.z = (nz + 4 + ga.chunk - 1) / ga.chunk;
     const int k = run.prof_begin("remap_sweep_geom_march", 0, 8, (double)(nx + 4) * (ny + 4) * (nz + 4));
     k_geom_march<A, R><<<grd, blk, 0, run.s>>>(ga);
     run.prof_end(k);
@@ -1530,7 +1535,9 @@ void remap_sweep(Run<R>& run, bool predictor, int dt_slot, int pass[3], int bmod
       dim3 grd((nx + 4 + kMEXOut - 1) / kMEXOut, (ny + 4 + 3) / 4, nz + 4);
       k_mass_energy_x<R><<<grd, blk, 0, run.s>>>(me, sx, sxy, nx);
     } else {
-      dim3 grd((nt1 + 4 + 31) / 32, (nt2 + 4 + 3) / 4, (na + 4 + kMEChunk - 1) / kMEChunk);
+      dim3 grd((nt1 + 4 + 31) / 32, (nt2 + 4 + 3) / 4, 1);
+      me.chunk = march_chunk(na + 4, grd.x * grd.y, kMEChunk, resident_blocks<k_mass_energy_march<R>>(128));
+      grd.z = (na + 4 + me.chunk - 1) / me.chunk;
       k_mass_energy_march<R><<<grd, blk, 0, run.s>>>(me);
     }
     run.prof_end(k);
@@ -1626,7 +1633,9 @@ void remap_sweep(Run<R>& run, bool predictor, int dt_slot, int pass[3], int bmod
         dim3 grd((nx + 1 + kVMXOut - 1) / kVMXOut, (ny + 1 + 3) / 4, nz + 1);
         k_vm_x<R><<<grd, dim3(32, 4, 1), 0, run.s>>>(vm);
       } else {
-        dim3 grd((nx + 1 + 31) / 32, (gm.n3 + 1 + 3) / 4, (na + 1 + kMomA - 1) / kMomA);
+        dim3 grd((nx + 1 + 31) / 32, (gm.n3 + 1 + 3) / 4, 1);
+        vm.m.chunk = march_chunk(na + 1, grd.x * grd.y, kMomA, resident_blocks<k_vm_march<A, R>>(128));
+        grd.z = (na + 1 + vm.m.chunk - 1) / vm.m.chunk;
         k_vm_march<A, R><<<grd, dim3(32, 4, 1), 0, run.s>>>(vm);
       }
     } else if (A == 0) {
@@ -1636,7 +1645,9 @@ void remap_sweep(Run<R>& run, bool predictor, int dt_slot, int pass[3], int bmod
       else
         k_mom_x<R, false><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
     } else {
-      dim3 grd((nx + 1 + 31) / 32, (gm.n3 + 1 + 3) / 4, (na + 1 + kMomA - 1) / kMomA);
+      dim3 grd((nx + 1 + 31) / 32, (gm.n3 + 1 + 3) / 4, 1);
+      gm.chunk = march_chunk(na + 1, grd.x * grd.y, kMomA, resident_blocks<k_mom_march<R, true>>(128));
+      grd.z = (na + 1 + gm.chunk - 1) / gm.chunk;
       if (rke)
         k_mom_march<R, true><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
       else

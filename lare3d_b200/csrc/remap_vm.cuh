@@ -121,8 +121,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 4 : 6) k_vm_march(VMArgs
   const int t0 = (int)(blockIdx.x * blockDim.x + threadIdx.x);  // x, 0..nx
   const int t1 = (int)(blockIdx.y * blockDim.y + threadIdx.y);  // the third axis, 0..n3
   if (t0 > g.nx || t1 > g.n3) return;
-  const int ia0 = (int)blockIdx.z * kMomA;
-  const int ia1 = min(ia0 + kMomA - 1, g.na);
+  const int ia0 = (int)blockIdx.z * g.chunk;
+  const int ia1 = min(ia0 + g.chunk - 1, g.na);
   const R dt = (R)g.sc[g.dt_slot];
   const int SA = g.SA, S3 = g.S3;
   const int o[4] = {0, 1, S3, 1 + S3};
