@@ -31,6 +31,24 @@ struct A1 {
   __device__ __forceinline__ R operator()(int i) const { return p[i]; }
 };
 
+// Elements by their byte offset from an array's first element, Fortran
+// (-2, -2, -2).  All arrays share one layout, so one 32-bit offset serves
+// every array at a point, where an element index costs a 64-bit multiply-add
+// per array.  It cannot overflow: a context holds more than 50 arrays, so on
+// a GPU of less than 200 GB one array stays below 2^32 bytes.
+template <class R>
+__device__ __forceinline__ unsigned elem_off(int i, int si, int j, int sj) {
+  return (unsigned)((i + 2) * si + (j + 2) * sj) * (unsigned)sizeof(R);
+}
+template <class R>
+__device__ __forceinline__ R elem_at(const R* first, unsigned off) {
+  return __ldg(reinterpret_cast<const R*>(reinterpret_cast<const char*>(first) + off));
+}
+template <class R>
+__device__ __forceinline__ R& elem_ref(R* first, unsigned off) {
+  return *reinterpret_cast<R*>(reinterpret_cast<char*>(first) + off);
+}
+
 template <class R>
 struct Num;
 template <>

@@ -125,6 +125,7 @@ struct Run {
   int peak_substeps = 0, last_substeps = 0, steps_taken = 0, n_s_stages = 0;
   int blk_x = 32, blk_y = 4;            // block shape of the point kernels (measured best at 256^3)
   bool capturing = false;               // recording a CUDA graph of whole steps
+  bool launch_error = false;            // a tensor map could not be made
   cudaStream_t s_body = nullptr;        // captures the body of the resistive sub-cycle loop
   GSpec g_cell, g_node, g_bx, g_by, g_bz, g_cell_mpi, g_cell_user, g_dm[3];
   Prof prof;
@@ -762,6 +763,44 @@ __device__ __forceinline__ LimOut<R> limiter_dv(R v_advect, R fm, R fi, R fp, R 
   L.Di = L.sign_v * ss * fmin(fmin(fabs(Da) * L.dxbu, fabs(dfi)), fabs(dfu));
   return L;
 }
+#if LARE_FAST
+// The product build's limited flux per unit mass or area moved, in terms of
+// the faces' differences d and slopes s = |d| / dxc (faces below, at and
+// above c): the reference's expressions regrouped, with the upwind choices
+// (whose weights are exactly 0 or 1) and the product of signs taken by
+// selection.  phi = |v dt| * rxu; the result is (f_u + D (1 - phi)) v dt.
+template <class R>
+__device__ __forceinline__ R lesser(R a, R b) {
+  return a < b ? a : b;
+}
+template <>
+__device__ __forceinline__ float lesser(float a, float b) {
+  return fminf(a, b);
+}
+// copies +-m: zero unless a and b have the same sign, else m with the sign of a * s
+__device__ __forceinline__ double signed_min(double m, double a, double b, double s) {
+  const int ha = __double2hiint(a);
+  const bool same = (ha ^ __double2hiint(b)) >= 0;
+  const int h = __double2hiint(m) | ((ha ^ __double2hiint(s)) & 0x80000000);
+  return same ? __hiloint2double(h, __double2loint(m)) : 0.0;
+}
+__device__ __forceinline__ float signed_min(float m, float a, float b, float s) {
+  const int ha = __float_as_int(a);
+  const bool same = (ha ^ __float_as_int(b)) >= 0;
+  return same ? __int_as_float(__float_as_int(m) | ((ha ^ __float_as_int(s)) & 0x80000000)) : 0.0f;
+}
+template <class R>
+__device__ __forceinline__ R van_leer(R v, R vdt, R f0, R fp, R dm, R d0, R dp, R sm, R s0, R sp, R db0, R dbp, R r0,
+                                      R rp) {
+  const bool up = !signbit(v);
+  const R phi = fabs(vdt) * (up ? r0 : rp);
+  const R du = up ? dm : dp;
+  const R da = (R(2) - phi) * s0 + (R(1) + phi) * (up ? sm : sp);
+  const R m = lesser(lesser(fabs(da) * ((up ? db0 : dbp) * (R(1) / R(6))), R(fabs(d0))), R(fabs(du)));
+  const R D = signed_min(m, d0, du, v);
+  return ((up ? f0 : fp) + D * (R(1) - phi)) * vdt;
+}
+#endif
 // The same with plain divisors.
 template <class R>
 __device__ __forceinline__ LimOut<R> limiter(R v_advect, R fm, R fi, R fp, R fp2, R dxci, R dxcm, R dxcp, R dxbi,
@@ -776,6 +815,12 @@ LARE_END  // namespace lare
 
 LARE_BEGIN
 
+// The axes of a step's three sweeps in order (remap.f90:71-99).
+inline const int* sweep_order(int step) {
+  static const int order[6][3] = {{0, 1, 2}, {1, 2, 0}, {2, 0, 1}, {0, 2, 1}, {2, 1, 0}, {1, 0, 2}};
+  return order[((step % 6) + 6) % 6];
+}
+
 // remap.f90:33-131 eulerian_remap (the corrector's full remap; the
 // predictor's B-only remap is predictor_remap in lagran.cuh).
 template <class R>
@@ -789,14 +834,13 @@ void eulerian_remap(Run<R>& run, int step) {
   }
   // B -> flux form (remap.f90:43-69) and back (:101-127) are done by the
   // first and last sweeps' B kernels on the way (remap_sweep's bmode).
-  static const int order[6][3] = {{0, 1, 2}, {1, 2, 0}, {2, 0, 1}, {0, 2, 1}, {2, 1, 0}, {1, 0, 2}};
-  int cse = ((step % 6) + 6) % 6;
+  const int* const order = sweep_order(step);
   for (int s = 0; s < 3; ++s) {
     const int bmode = s == 0 ? 1 : (s == 2 ? 2 : 0);
-    switch (order[cse][s]) {
-      case 0: remap_sweep<0>(run, false, SC_DT, pass, bmode); break;
-      case 1: remap_sweep<1>(run, false, SC_DT, pass, bmode); break;
-      default: remap_sweep<2>(run, false, SC_DT, pass, bmode); break;
+    switch (order[s]) {
+      case 0: remap_sweep<0>(run, SC_DT, pass, bmode); break;
+      case 1: remap_sweep<1>(run, SC_DT, pass, bmode); break;
+      default: remap_sweep<2>(run, SC_DT, pass, bmode); break;
     }
   }
   bfield_bcs(run);

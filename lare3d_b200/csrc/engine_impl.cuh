@@ -85,6 +85,7 @@ class EngineT : public EngineBase {
   int cuda_check(const char* where) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(LARE_ECUDA, std::string(where) + ": " + cudaGetErrorString(e));
+    if (run.launch_error) return fail(LARE_ECUDA, std::string(where) + ": tensor map");
     return LARE_OK;
   }
 
@@ -189,13 +190,17 @@ class EngineT : public EngineBase {
     long long sxy = (long long)run.sx * sy;
     long long elems = sxy * sz;
     if (elems >= (1LL << 31)) { err = "grid too large for 32-bit indexing"; return LARE_EINVAL; }
+    // byte offsets within an array are 32-bit (elem_at): an array past that
+    // is one of more than 50, which no GPU of less than 200 GB holds
+    if (elems * (long long)sizeof(R) >= (1LL << 32)) { err = "cudaMalloc: an array of 4 GiB or more"; return LARE_ENOMEM; }
     run.sxy = (int)sxy;
     run.elems = (size_t)elems;
     const long long off = 2 + 2LL * run.sx + 2LL * sxy;
     if (cudaStreamCreateWithFlags(&run.s, cudaStreamNonBlocking) != cudaSuccess) { err = "stream"; return LARE_ECUDA; }
     // kernels with more than the default 48 KiB of dynamic shared memory
     if (cudaFuncSetAttribute(k_lp4_tile<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lp4_smem_bytes<R>()) !=
-        cudaSuccess) {
+            cudaSuccess ||
+        bs_attributes<R>() != cudaSuccess) {
       err = "shared memory attribute";
       return LARE_ECUDA;
     }
@@ -638,6 +643,7 @@ class EngineT : public EngineBase {
   }
   int scalars(lare_scalars* o) override {
     if (pull_scalars(run) != cudaSuccess) return fail(LARE_ECUDA, "scalars: sync failed");
+    if ((int)run.host_sc[SC_ERROR] == LARE_ECUDA) return fail(LARE_ECUDA, "a tile copy never arrived");
     o->time = run.host_sc[SC_TIME];
     o->dt = run.host_sc[SC_DT];
     o->dtr = run.host_sc[SC_DTR];

@@ -579,35 +579,32 @@ void set_dt(Run<R>& run) {
 template <class R>
 void predictor_remap(Run<R>& run, int step) {
   Arrays<R>& A = run.a;
-  // B -> flux form (remap.f90:43-69, into the B0 buffers, which are then
-  // swapped in so that B itself is kept as B0) and back (:101-127) are done
-  // by the first and last sweeps' B kernels on the way (remap_sweep's bmode).
-  // vx1 = vx (lagran.F90:1051-1053): the sweeps read v itself.  vx1's own
-  // nodes 0:n are rewritten by the predictor force and its ghosts by
-  // remap_v_bcs, except on an open side: there the copy's ghost values are
-  // carried into the vx1 buffer.
+  // The sweeps carry B from the step's arrays through the B0 and B1 buffers
+  // (the first puts it in flux form, the last back: remap.f90:43-69, :101-127),
+  // so B itself is kept as B0.  vx1 = vx (lagran.F90:1051-1053): the sweeps
+  // read v itself.  vx1's own nodes 0:n are rewritten by the predictor force
+  // and its ghosts by remap_v_bcs, except on an open side: there the copy's
+  // ghost values are carried into the vx1 buffer.
   R* const keep[3] = {A.vx1.p, A.vy1.p, A.vz1.p};
-  {
-    R* const ov[3] = {A.vx.p, A.vy.p, A.vz.p};
-    carry_velocity(run, keep, ov);
-  }
-  A.vx1.p = A.vx.p;
-  A.vy1.p = A.vy.p;
-  A.vz1.p = A.vz.p;
-  static const int order[6][3] = {{0, 1, 2}, {1, 2, 0}, {2, 0, 1}, {0, 2, 1}, {2, 1, 0}, {1, 0, 2}};
-  int cse = ((step % 6) + 6) % 6;
-  int pass[3] = {1, 1, 1};
+  R* const v[3] = {A.vx.p, A.vy.p, A.vz.p};
+  carry_velocity(run, keep, v);
+  R* const b[3] = {A.bx.p, A.by.p, A.bz.p};
+  R* const p[3] = {A.bx0.p, A.by0.p, A.bz0.p};
+  R* const q[3] = {A.bx1.p, A.by1.p, A.bz1.p};
+  const int* const order = sweep_order(step);
   for (int s = 0; s < 3; ++s) {
     const int bmode = s == 0 ? 1 : (s == 2 ? 2 : 0);
-    switch (order[cse][s]) {
-      case 0: remap_sweep<0>(run, true, SC_DT2, pass, bmode); break;
-      case 1: remap_sweep<1>(run, true, SC_DT2, pass, bmode); break;
-      default: remap_sweep<2>(run, true, SC_DT2, pass, bmode); break;
+    R* const(&in)[3] = s == 0 ? b : (s == 1 ? p : q);
+    R* const(&out)[3] = s == 1 ? q : p;
+    switch (order[s]) {
+      case 0: bsweep<0>(run, v[0], in, out, SC_DT2, bmode); break;
+      case 1: bsweep<1>(run, v[1], in, out, SC_DT2, bmode); break;
+      default: bsweep<2>(run, v[2], in, out, SC_DT2, bmode); break;
     }
   }
-  A.vx1.p = keep[0];
-  A.vy1.p = keep[1];
-  A.vz1.p = keep[2];
+  std::swap(A.bx.p, A.bx0.p);
+  std::swap(A.by.p, A.by0.p);
+  std::swap(A.bz.p, A.bz0.p);
   bfield_bcs(run);
 }
 
@@ -753,17 +750,36 @@ void predictor_corrector_step(Run<R>& run) {
   R* const energy = A.energy.p;
   const R* energy0 = A.energy0.p;
   R* const pressure = A.pressure.p;
-  const R* cv1 = A.cv1.p;
+  R* const cv1 = A.cv1.p;
   const R* cv = A.cv.p;
   const R* rho = A.rho.p;
   const R* visc_heat = A.visc_heat.p;
+  R* const vx = A.vx.p;
+  R* const vy = A.vy.p;
+  R* const vz = A.vz.p;
+  // cv1 is the predictor's last sweep's, whose terms add in its axis' order
+  const int last_axis = sweep_order(run.cur_step)[2];
+  auto mx = A.dxb, my = A.dyb, mz = A.dzb;
+  const A1<R> rmx = A.rdb[0], rmy = A.rdb[1], rmz = A.rdb[2];
   const bool cond = run.p.conduction != 0;
   const R* erad = run.p.radiation ? A.erad.p : nullptr;  // the energy after rad_losses
   const R g = (R)run.p.gamma, xi = (R)run.p.xi_n, ip = (R)run.p.ionise_pot;
   const R* xin = run.pip ? A.xi.p : nullptr;
   const double* sc = run.sc;
-  LARE_BOXWH(run, 0, 4, 8, -1, nx + 2, -1, ny + 2, -1, nz + 2, [=] __device__(int ix, int iy, int iz) {
+  LARE_BOXWH(run, 0, 4, 11, -1, nx + 2, -1, ny + 2, -1, nz + 2, [=] __device__(int ix, int iy, int iz) {
+    const R dt2 = (R)sc[SC_DT2];
     const int c = ix + sx * iy + sxy * iz;
+    // the volume after the half step, from the face velocities (xremap.f90:64-86)
+    auto vxf = [&](int q) { return (vx[q] + vx[q - sx] + vx[q - sxy] + vx[q - sx - sxy]) * R(0.25); };
+    auto vyf = [&](int q) { return (vy[q] + vy[q - 1] + vy[q - sxy] + vy[q - 1 - sxy]) * R(0.25); };
+    auto vzf = [&](int q) { return (vz[q] + vz[q - 1] + vz[q - sx] + vz[q - 1 - sx]) * R(0.25); };
+    const R tx = div_rcp(vxf(c) - vxf(c - 1), mx(ix), rmx(ix));
+    const R ty = div_rcp(vyf(c) - vyf(c - sx), my(iy), rmy(iy));
+    const R tz = div_rcp(vzf(c) - vzf(c - sxy), mz(iz), rmz(iz));
+    const R tt = last_axis == 0 ? ty + tz + tx : (last_axis == 1 ? tx + tz + ty : tx + ty + tz);
+    const R cvc = cv[c];
+    const R cv1c = cvc * (R(1) + tt * dt2);
+    cv1[c] = cv1c;
     R e;
     if (cond) {
       R e0 = energy0[c];
@@ -780,13 +796,12 @@ void predictor_corrector_step(Run<R>& run) {
     e = e > R(0) ? e : R(0);
     energy[c] = e;
     if (ix >= 0 && ix <= nx + 1 && iy >= 0 && iy <= ny + 1 && iz >= 0 && iz <= nz + 1) {
-      const R dt2 = (R)sc[SC_DT2];
       const R rr = dv_of(rho[c]);
-      R dv = qdiv(cv1[c], cv[c]) - R(1);
+      R dv = qdiv(cv1c, cvc) - R(1);
       R e1 = e - dv_div(pressure[c] * dv, rr);
       e1 = e1 + dv_div(visc_heat[c] * dt2, rr);
       const R x = xin ? xin[c] : xi;
-      pressure[c] = qdiv((e1 - (R(1) - x) * ip) * (g - R(1)) * rho[c] * cv[c], cv1[c]);
+      pressure[c] = qdiv((e1 - (R(1) - x) * ip) * (g - R(1)) * rho[c] * cvc, cv1c);
     }
   });
   // PC2 (0:n): vertex forces with the predicted B; half-step velocity
@@ -795,9 +810,6 @@ void predictor_corrector_step(Run<R>& run) {
   const R* bz = A.bz.p;
   const R* gamma_boris = A.gamma_boris.p;
   const R* rho_v = A.rho_v.p;
-  R* const vx = A.vx.p;
-  R* const vy = A.vy.p;
-  R* const vz = A.vz.p;
   R* const vx1 = A.vx1.p;
   R* const vy1 = A.vy1.p;
   R* const vz1 = A.vz1.p;

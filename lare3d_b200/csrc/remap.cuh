@@ -3,18 +3,16 @@
 // xremap.f90:37-336 remap_x and its mirrors yremap.f90:37-337 and
 // zremap.f90:37-336, for a sweep along axis A (0 = x, 1 = y, 2 = z).  The
 // reference runs about 25 loop nests per sweep; here they are grouped into
-// eight kernels.  Every element is still computed by exactly the reference's
+// a few kernels.  Every element is still computed by exactly the reference's
 // expression over exactly the same inputs, so the results are unchanged bit
 // for bit; what changes is where intermediates live:
 //
 //   K1 geometry   cv1, cv2, dxb1 and dxc1 (xremap.f90:57-115); dxb1 at p+e_A
 //                 is recomputed in the thread for dxc1.
-//   K2 B fluxes   both constrained-transport edge fluxes (:340-470); the
-//                 second does not read what the first one's updates change.
-//                 The y and z sweeps use a marching kernel and the x sweep
-//                 a warp-shuffle kernel; both form each quotient once.
-//   K3 B update   the four flux-difference updates (:121-157), with each
-//                 file's own loop ranges as predicates.
+//   K2 B          both constrained-transport edge fluxes (:340-470) and the
+//                 four flux-difference updates (:121-157) with the geometry
+//                 they need, one kernel (remap_b.cuh) into a second set of B
+//                 arrays.
 //   K4 mass flux  dm (:474-533) over the whole cell box, with dm_x_bcs
 //                 (:899-917) folded in: a ghost element is the flux computed
 //                 at its source index (the same value the copy would bring).
@@ -27,11 +25,7 @@
 //                 kernel that writes the new velocities to second buffers.
 // The face-averaged vx1 written back at :265 is only read again as
 // REAL(xpass)*(...) with xpass = 0, so it is formed in K8 and not stored.
-// Predictor sweeps (predictor_step = .TRUE.) stop after K3.
-// B's conversion to flux form before a remap's three sweeps
-// (remap.f90:43-69) and back after them (:101-127) happens in the first
-// sweep's K2 and K3 and the last sweep's K3 (remap_sweep's bmode), not in
-// passes of their own.
+// The predictor's sweeps (predictor_step = .TRUE.) are K2 alone.
 //
 // Indexing is linear: c = ix + sx*iy + sxy*iz, neighbours by constant
 // offsets, with the axis a compile-time parameter.
@@ -39,355 +33,9 @@
 
 #include <utility>
 
+#include "remap_b.cuh"
+
 LARE_BEGIN
-
-template <int A>
-__device__ __forceinline__ int acoord(int ix, int iy, int iz) {
-  return A == 0 ? ix : (A == 1 ? iy : iz);
-}
-
-// K2 for the y and z sweeps as a marching kernel.  A thread owns a run of
-// kMarch consecutive cells along the sweep axis A at one (x, transverse)
-// position and walks it, keeping the quotients B/dbv, the dbv and the db1
-// and dc1 values of the four-point stencil in registers: each step loads
-// the one new stencil point instead of all four and forms one quotient per
-// flux instead of four.  Every value is the same expression of the same
-// operands as in the per-cell form, so the fluxes are identical bit for bit.
-constexpr int kMarch = 32;
-constexpr int kBUpdZ32 = 4, kBUpdZ64 = 1;  // z-points per thread of the B updates (measured)
-
-template <class R>
-struct BfArgs {
-  const R* va;           // velocity component along A (v1 of the reference)
-  const R* b1;           // first transported component
-  const R* b2;           // second
-  const R* db1;
-  const R* dc1;
-  R* f1;
-  R* f2;
-  const double* sc;
-  int dt_slot;
-  int SA, SB1, SB2, SO1, SO2;  // strides along A, the two components' own axes, and their remaining axes
-  int SX, SY;                  // strides of the thread grid's two axes (x and the other transverse axis)
-  int na;                      // cells along A
-  int n0, n1;                  // extents of the thread grid (-1..n+1 each)
-  // for the first sweep of a remap, which reads B itself and forms its
-  // flux form on the fly: the metrics, the components' axes, the sweep axis
-  A1<R> dbm[3];
-  int j1, j2, ax;
-};
-
-// remap.f90:43-69 on one value: B component j at (ix, iy, iz) times the
-// widths of its face along the other two axes, in axis order, where the
-// reference converts (its B arrays start at -1 on the other axes).
-template <class R>
-__device__ __forceinline__ R to_flux(R b, int j, int ix, int iy, int iz, const A1<R> (&m)[3]) {
-  if (j == 0) return (iy >= -1 && iz >= -1) ? b * m[1](iy) * m[2](iz) : b;
-  if (j == 1) return (ix >= -1 && iz >= -1) ? b * m[0](ix) * m[2](iz) : b;
-  return (ix >= -1 && iy >= -1) ? b * m[0](ix) * m[1](iy) : b;
-}
-// remap.f90:101-127 on one value: the flux form back to B.
-template <class R>
-__device__ __forceinline__ R from_flux(R b, int j, int ix, int iy, int iz, const A1<R> (&m)[3],
-                                       const A1<R> (&r)[3]) {
-  if (j == 0) return (iy >= -1 && iz >= -1) ? div_rcp(div_rcp(b, m[1](iy), r[1](iy)), m[2](iz), r[2](iz)) : b;
-  if (j == 1) return (ix >= -1 && iz >= -1) ? div_rcp(div_rcp(b, m[0](ix), r[0](ix)), m[2](iz), r[2](iz)) : b;
-  return (ix >= -1 && iy >= -1) ? div_rcp(div_rcp(b, m[0](ix), r[0](ix)), m[1](iy), r[1](iy)) : b;
-}
-
-// to_flux along a y/z-sweep march line (the first sweep of a remap): the
-// line's points have every coordinate >= -1, so the reference converts them
-// all; of component j's two face widths, the one across the line (axis c =
-// 3 - j - A, at the thread's x or second grid coordinate) is fixed and is
-// formed once, the one along the sweep axis is loaded per point and shared
-// by both components; they multiply in axis order as in remap.f90:43-69.
-template <class R>
-struct LineConv {
-  const R* mA;  // widths along the sweep axis
-  R cf1, cf2;   // the fixed widths of the two components
-  bool af1, af2;  // the sweep axis comes first
-};
-template <class R>
-__device__ __forceinline__ LineConv<R> line_conv(const BfArgs<R>& a, int x, int g2) {
-  LineConv<R> L;
-  L.mA = a.ax == 1 ? a.dbm[1].p : a.dbm[2].p;
-  const int ay = 3 - a.ax;  // the grid's second axis: z for the y sweep, y for the z sweep
-  auto fixed = [&](int j) {
-    const int c = 3 - j - a.ax;
-    return c == 0 ? a.dbm[0](x) : (ay == 1 ? a.dbm[1](g2) : a.dbm[2](g2));
-  };
-  L.cf1 = fixed(a.j1);
-  L.cf2 = fixed(a.j2);
-  L.af1 = a.ax < 3 - a.j1 - a.ax;
-  L.af2 = a.ax < 3 - a.j2 - a.ax;
-  return L;
-}
-template <class R>
-__device__ __forceinline__ R line_form(R b, R ma, R cf, bool afirst) {
-  return afirst ? b * ma * cf : b * cf * ma;
-}
-
-// B / dbv at q, with dbv (in the carried divisor form dv_of) returned in dvb
-template <class R>
-__device__ __forceinline__ R bf_quot(R b, const R* db1, int q, int SB, R& dvb) {
-  dvb = dv_of((db1[q] + db1[q + SB]) * R(0.5));
-  return dv_div(b, dvb);
-}
-
-template <class R, bool PRE>
-__global__ void __launch_bounds__(256, 2) k_bflux_march(BfArgs<R> a) {
-  const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
-  const int t1 = blockIdx.y * blockDim.y + threadIdx.y;
-  if (t0 >= a.n0 || t1 >= a.n1) return;
-  const int ia0 = -1 + (int)blockIdx.z * kMarch;
-  const int ia1 = min(ia0 + kMarch - 1, a.na + 1);
-  const int SA = a.SA;
-  // cell (t0 - 1, t1 - 1, ia0) in grid / along-A coordinates
-  int c = (t0 - 1) * a.SX + (t1 - 1) * a.SY + ia0 * SA;
-  const R dt = (R)a.sc[a.dt_slot];
-  // four-point windows at cm, c, cp, cp2 (clamped as MAX(ia-1,-1), MIN(ia+2,na+2))
-  R q1m, q10, q1p, q1p2, d1m, d10, d1p, d1p2;  // flux 1: quotients, dbv
-  R q2m, q20, q2p, q2p2, d2m, d20, d2p, d2p2;  // flux 2
-  R dcm, dc0, dcp, dbc0, dbcp;                 // dc1 at cm, c, cp; db1 at c, cp
-  const int gx = t0 - 1, g2 = t1 - 1;  // the thread grid's coordinates
-  LineConv<R> lc{};
-  if constexpr (PRE) lc = line_conv(a, gx, g2);
-  {
-    const int am = ia0 > -1 ? ia0 - 1 : ia0, ap2 = ia0 + 2 <= a.na + 2 ? ia0 + 2 : ia0 + 1;
-    const int cm = c + (am - ia0) * SA;
-    const int cp = c + SA;
-    const int cp2 = c + (ap2 - ia0) * SA;
-    auto b1 = [&](int q, int ia) {
-      if constexpr (PRE) return line_form(a.b1[q], lc.mA[ia], lc.cf1, lc.af1);
-      return a.b1[q];
-    };
-    auto b2 = [&](int q, int ia) {
-      if constexpr (PRE) return line_form(a.b2[q], lc.mA[ia], lc.cf2, lc.af2);
-      return a.b2[q];
-    };
-    q1m = bf_quot(b1(cm, am), a.db1, cm, a.SB1, d1m);
-    q10 = bf_quot(b1(c, ia0), a.db1, c, a.SB1, d10);
-    q1p = bf_quot(b1(cp, ia0 + 1), a.db1, cp, a.SB1, d1p);
-    q1p2 = bf_quot(b1(cp2, ap2), a.db1, cp2, a.SB1, d1p2);
-    q2m = bf_quot(b2(cm, am), a.db1, cm, a.SB2, d2m);
-    q20 = bf_quot(b2(c, ia0), a.db1, c, a.SB2, d20);
-    q2p = bf_quot(b2(cp, ia0 + 1), a.db1, cp, a.SB2, d2p);
-    q2p2 = bf_quot(b2(cp2, ap2), a.db1, cp2, a.SB2, d2p2);
-    dcm = dv_of(a.dc1[cm]);
-    dc0 = dv_of(a.dc1[c]);
-    dcp = dv_of(a.dc1[cp]);
-    dbc0 = a.db1[c];
-    dbcp = a.db1[cp];
-  }
-  (void)d1m;
-  (void)d2m;
-  R va0 = a.va[c], va1 = a.va[c - a.SO1], va2 = a.va[c - a.SO2];
-  for (int ia = ia0; ia <= ia1; ++ia) {
-    // issue the next step's loads before this step's arithmetic
-    const int cn = c + SA;
-    const bool more = ia < ia1;
-    const bool clamp = ia + 3 > a.na + 2;
-    const int qn = cn + 2 * SA;
-    const bool fetch = more && !clamp;
-    R nb1 = R(0), nb2 = R(0), nd = R(0), nd1 = R(0), nd2 = R(0), ndc = R(0), ndb = R(0);
-    R nva0 = R(0), nva1 = R(0), nva2 = R(0);
-    if (fetch) {
-      nb1 = a.b1[qn];
-      nb2 = a.b2[qn];
-      if constexpr (PRE) {
-        const R ma = lc.mA[ia + 3];
-        nb1 = line_form(nb1, ma, lc.cf1, lc.af1);
-        nb2 = line_form(nb2, ma, lc.cf2, lc.af2);
-      }
-      nd = a.db1[qn];
-      nd1 = a.db1[qn + a.SB1];
-      nd2 = a.db1[qn + a.SB2];
-    }
-    if (more) {
-      ndc = a.dc1[cn + SA];
-      ndb = a.db1[cn + SA];
-    }
-    if (more) {
-      nva0 = a.va[cn];
-      nva1 = a.va[cn - a.SO1];
-      nva2 = a.va[cn - a.SO2];
-    }
-    {
-      const R v_advect = (va0 + va1) * R(0.5);
-      LimOut<R> L = limiter_dv<R>(v_advect, q1m, q10, q1p, q1p2, dc0, dcm, dcp, dbc0, dbcp, d10, d1p, dt, true);
-      a.f1[c] = (L.fu + L.Di * (R(1) - L.phi)) * v_advect * dt;
-    }
-    {
-      const R v_advect = (va0 + va2) * R(0.5);
-      LimOut<R> L = limiter_dv<R>(v_advect, q2m, q20, q2p, q2p2, dc0, dcm, dcp, dbc0, dbcp, d20, d2p, dt, true);
-      a.f2[c] = (L.fu + L.Di * (R(1) - L.phi)) * v_advect * dt;
-    }
-    if (!more) break;
-    q1m = q10; q10 = q1p; q1p = q1p2;
-    d10 = d1p; d1p = d1p2;
-    q2m = q20; q20 = q2p; q2p = q2p2;
-    d20 = d2p; d2p = d2p2;
-    if (clamp) {
-      q1p2 = q1p; d1p2 = d1p;
-      q2p2 = q2p; d2p2 = d2p;
-    } else {
-      d1p2 = dv_of((nd + nd1) * R(0.5));
-      q1p2 = dv_div(nb1, d1p2);
-      d2p2 = dv_of((nd + nd2) * R(0.5));
-      q2p2 = dv_div(nb2, d2p2);
-    }
-    dcm = dc0; dc0 = dcp; dcp = dv_of(ndc);
-    dbc0 = dbcp; dbcp = ndb;
-    va0 = nva0; va1 = nva1; va2 = nva2;
-    c = cn;
-  }
-}
-
-// K2 for the x sweep: the lanes of a warp hold consecutive x positions, and
-// the stencil neighbours along x (one to the left, two to the right) come
-// from the neighbouring lanes by shuffles, so a lane loads its own point
-// once and forms one quotient per flux.  A warp spans 32 positions and
-// writes the kXOut = 29 whose whole stencil lies inside it; warps overlap by
-// three positions.  Same expressions, same operands, same results bit for
-// bit as the per-cell form.  The launch bounds cap the FP64 form at 48
-// registers: it is latency-bound, and the extra resident warps outweigh the
-// few spills (measured at 256^3).
-constexpr int kXOut = 29;
-
-template <class R, bool PRE>
-__global__ void __launch_bounds__(128, 10) k_bflux_x(BfArgs<R> a, int sx, int sxy, int nx, int ny) {
-  const int lane = (int)threadIdx.x;                           // blockDim.x == 32: one warp per row
-  const int ix = -2 + (int)blockIdx.x * kXOut + lane;          // this lane's x position
-  const int iy = -1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-  const int iz = -1 + (int)blockIdx.z;
-  if (iy > ny + 1) return;                                      // uniform over the warp
-  const int cx = min(ix, nx + 2);
-  const int c = cx + sx * iy + sxy * iz;                        // positions past n+2 load n+2 (unused)
-  R d1, d2;
-  R bv1 = a.b1[c], bv2 = a.b2[c];
-  if constexpr (PRE) {  // the first sweep of a remap reads B itself (by and bz)
-    bv1 = to_flux(bv1, 1, cx, iy, iz, a.dbm);
-    bv2 = to_flux(bv2, 2, cx, iy, iz, a.dbm);
-  }
-  const R q1 = bf_quot(bv1, a.db1, c, a.SB1, d1);
-  const R q2 = bf_quot(bv2, a.db1, c, a.SB2, d2);
-  const R dc = dv_of(a.dc1[c]), db = a.db1[c];
-  const unsigned all = 0xffffffffu;
-  const R q1m = __shfl_up_sync(all, q1, 1), q1p = __shfl_down_sync(all, q1, 1), q1p2 = __shfl_down_sync(all, q1, 2);
-  const R q2m = __shfl_up_sync(all, q2, 1), q2p = __shfl_down_sync(all, q2, 1), q2p2 = __shfl_down_sync(all, q2, 2);
-  const R d1p = __shfl_down_sync(all, d1, 1), d2p = __shfl_down_sync(all, d2, 1);
-  const R dcm = __shfl_up_sync(all, dc, 1), dcp = __shfl_down_sync(all, dc, 1);
-  const R dbp = __shfl_down_sync(all, db, 1);
-  if (lane < 1 || lane > kXOut || ix > nx + 1) return;
-  const bool left = ix > -1;            // cm = MAX(ix - 1, -1)
-  const bool right = ix + 2 <= nx + 2;  // cp2 = MIN(ix + 2, n + 2)
-  const R dt = (R)a.sc[a.dt_slot];
-  const R va0 = a.va[c], va1 = a.va[c - a.SO1], va2 = a.va[c - a.SO2];
-  {
-    const R v_advect = (va0 + va1) * R(0.5);
-    LimOut<R> L = limiter_dv<R>(v_advect, left ? q1m : q1, q1, q1p, right ? q1p2 : q1p, dc, left ? dcm : dc, dcp, db,
-                             dbp, d1, d1p, dt, true);
-    a.f1[c] = (L.fu + L.Di * (R(1) - L.phi)) * v_advect * dt;
-  }
-  {
-    const R v_advect = (va0 + va2) * R(0.5);
-    LimOut<R> L = limiter_dv<R>(v_advect, left ? q2m : q2, q2, q2p, right ? q2p2 : q2p, dc, left ? dcm : dc, dcp, db,
-                             dbp, d2, d2p, dt, true);
-    a.f2[c] = (L.fu + L.Di * (R(1) - L.phi)) * v_advect * dt;
-  }
-}
-
-// The same march with one flux per thread: blockIdx.z selects the flux
-// (even: first, odd: second) and the chunk, so a thread carries one
-// four-point window instead of two; twice the threads, about half the
-// registers each.
-template <class R, bool PRE>
-__global__ void __launch_bounds__(128) k_bflux_march1(BfArgs<R> a) {
-  const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
-  const int t1 = blockIdx.y * blockDim.y + threadIdx.y;
-  if (t0 >= a.n0 || t1 >= a.n1) return;
-  const bool second = (blockIdx.z & 1u) != 0;
-  const int ia0 = -1 + (int)(blockIdx.z >> 1) * kMarch;
-  const int ia1 = min(ia0 + kMarch - 1, a.na + 1);
-  const int SA = a.SA;
-  const R* B = second ? a.b2 : a.b1;
-  const int SB = second ? a.SB2 : a.SB1;
-  const int SO = second ? a.SO2 : a.SO1;
-  R* const fo = second ? a.f2 : a.f1;
-  const int gx = t0 - 1, g2 = t1 - 1;  // the thread grid's coordinates
-  R cf = R(0);
-  bool af = false;
-  const R* mA = nullptr;
-  if constexpr (PRE) {
-    const LineConv<R> lc = line_conv(a, gx, g2);
-    cf = second ? lc.cf2 : lc.cf1;
-    af = second ? lc.af2 : lc.af1;
-    mA = lc.mA;
-  }
-  int c = gx * a.SX + g2 * a.SY + ia0 * SA;
-  const R dt = (R)a.sc[a.dt_slot];
-  R qm, q0, qp, qp2, dm, d0, dp, dp2;  // quotients and dbv at cm, c, cp, cp2
-  R dcm, dc0, dcp, dbc0, dbcp;
-  {
-    const int am = ia0 > -1 ? ia0 - 1 : ia0, ap2 = ia0 + 2 <= a.na + 2 ? ia0 + 2 : ia0 + 1;
-    const int cm = c + (am - ia0) * SA;
-    const int cp = c + SA;
-    const int cp2 = c + (ap2 - ia0) * SA;
-    auto b = [&](int q, int ia) {
-      if constexpr (PRE) return line_form(B[q], mA[ia], cf, af);
-      return B[q];
-    };
-    qm = bf_quot(b(cm, am), a.db1, cm, SB, dm);
-    q0 = bf_quot(b(c, ia0), a.db1, c, SB, d0);
-    qp = bf_quot(b(cp, ia0 + 1), a.db1, cp, SB, dp);
-    qp2 = bf_quot(b(cp2, ap2), a.db1, cp2, SB, dp2);
-    dcm = dv_of(a.dc1[cm]);
-    dc0 = dv_of(a.dc1[c]);
-    dcp = dv_of(a.dc1[cp]);
-    dbc0 = a.db1[c];
-    dbcp = a.db1[cp];
-  }
-  (void)dm;
-  R va = a.va[c], vo = a.va[c - SO];
-  for (int ia = ia0; ia <= ia1; ++ia) {
-    const int cn = c + SA;
-    const bool more = ia < ia1;
-    const bool clamp = ia + 3 > a.na + 2;
-    const int qn = cn + 2 * SA;
-    const bool fetch = more && !clamp;
-    R nb = R(0), nd = R(0), nds = R(0), ndc = R(0), ndb = R(0), nva = R(0), nvo = R(0);
-    if (fetch) {
-      nb = B[qn];
-      if constexpr (PRE) nb = line_form(nb, mA[ia + 3], cf, af);
-      nd = a.db1[qn];
-      nds = a.db1[qn + SB];
-    }
-    if (more) {
-      ndc = a.dc1[cn + SA];
-      ndb = a.db1[cn + SA];
-    }
-    if (more) {
-      nva = a.va[cn];
-      nvo = a.va[cn - SO];
-    }
-    const R v_advect = (va + vo) * R(0.5);
-    LimOut<R> L = limiter_dv<R>(v_advect, qm, q0, qp, qp2, dc0, dcm, dcp, dbc0, dbcp, d0, dp, dt, true);
-    fo[c] = (L.fu + L.Di * (R(1) - L.phi)) * v_advect * dt;
-    if (!more) break;
-    qm = q0; q0 = qp; qp = qp2;
-    d0 = dp; dp = dp2;
-    if (clamp) {
-      qp2 = qp; dp2 = dp;
-    } else {
-      dp2 = dv_of((nd + nds) * R(0.5));
-      qp2 = dv_div(nb, dp2);
-    }
-    dcm = dc0; dc0 = dcp; dcp = dv_of(ndc);
-    dbc0 = dbcp; dbcp = ndb;
-    va = nva; vo = nvo;
-    c = cn;
-  }
-}
 
 // K1 as a z-marching kernel: a thread owns an (x, y) column and walks a
 // chunk of z.  Each face average (xremap.f90:64-86) sums two values of its
@@ -413,7 +61,6 @@ struct GeomArgs {
   const double* sc;
   int dt_slot, nx, ny, nz, sx, sxy;
   int chunk;
-  bool write_cv2;
 };
 
 template <int A, class R>
@@ -537,10 +184,8 @@ __global__ void __launch_bounds__(128) k_geom_march(GeomArgs<R> g) {
     R dv = (term_t1 + term_t2 + term_a) * dt;
     const R cvc = cur.cv;
     cv1_r[c] = cvc * (R(1) + dv);
-    if (g.write_cv2) {
-      dv = (term_t1 + term_t2) * dt;
-      cv2_r[c] = cvc * (R(1) + dv);
-    }
+    dv = (term_t1 + term_t2) * dt;
+    cv2_r[c] = cvc * (R(1) + dv);
     const R d0 = g.dbm[A](pp[A]) + dvv[A] * dt;
     db1_r[c] = d0;
     R d1 = d0;
@@ -903,108 +548,6 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 4 : 8) k_mom_march(MomAr
   }
 }
 
-// K3 with kBUpdZ z-points per thread: every load of all the thread's
-// points is issued before any store (a point reads and writes B only at
-// itself), so each thread keeps several independent loads in flight; the
-// FP32 form, 4 bytes a word, is otherwise latency-bound well below HBM
-// speed.  Same expressions and predicates as the per-point form.
-//
-// MODE 0, a middle sweep: the update in place over the box 0..n+1.
-// MODE 1, the first sweep of a remap: B is read as stored, put in flux form
-// (remap.f90:43-69) and updated over 0..n+1; every point of the arrays' box
-// -2..n+2 is written, to the output arrays (the predictor's B0 buffers,
-// whose B is kept, or B itself).  MODE 2, the last sweep: updated over
-// 0..n+1, then every point of -2..n+2 is put back from flux form
-// (remap.f90:101-127).  The conversions are the reference's expressions on
-// the same operands, so the result equals converting in separate passes.
-template <class R>
-struct BUpdArgs {
-  const R* f1;
-  const R* f2;
-  R* Ba;   // B along the sweep axis
-  R* Bb1;  // the two transported components
-  R* Bb2;
-  R* oa;   // where MODE 1 writes them
-  R* ob1;
-  R* ob2;
-  A1<R> dbm[3], rdbm[3];
-  int nx, ny, nz, sx, sxy, SA, SB1, SB2;
-};
-
-template <int A, int PTS, int MODE, class R>
-__global__ void __launch_bounds__(128) k_bupdate(BUpdArgs<R> g) {
-  constexpr int JA = A, J1 = A == 0 ? 1 : 0, J2 = A == 2 ? 1 : 2;  // the components' axes
-  constexpr int LO = MODE == 0 ? 0 : -2, EXT = MODE == 0 ? 1 : 2;   // the box LO..n+EXT
-  const int ix = LO + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int iy = LO + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-  if (ix > g.nx + EXT || iy > g.ny + EXT) return;
-  const int z0 = LO + (int)blockIdx.z * PTS;
-  const bool in_xy = ix >= 0 && ix <= g.nx + 1 && iy >= 0 && iy <= g.ny + 1;
-  R b1[PTS], f1c[PTS], f1a[PTS], ba[PTS], f1b[PTS], b2[PTS], f2c[PTS], f2a[PTS], f2b[PTS];
-  bool ok[PTS], in[PTS];
-#pragma unroll
-  for (int p = 0; p < PTS; ++p) {
-    const int iz = z0 + p;
-    ok[p] = iz <= g.nz + EXT;
-    in[p] = in_xy && iz >= 0 && iz <= g.nz + 1;  // the update box
-    const int c = ix + g.sx * iy + g.sxy * (ok[p] ? iz : z0);
-    b1[p] = g.Bb1[c];
-    ba[p] = g.Ba[c];
-    b2[p] = g.Bb2[c];
-    f1c[p] = f1a[p] = f1b[p] = f2c[p] = f2a[p] = f2b[p] = R(0);
-    if (in[p]) {
-      f1c[p] = g.f1[c];
-      f1a[p] = g.f1[c - g.SA];
-      f1b[p] = g.f1[c - g.SB1];
-      f2c[p] = g.f2[c];
-      f2a[p] = g.f2[c - g.SA];
-      f2b[p] = g.f2[c - g.SB2];
-    }
-  }
-#pragma unroll
-  for (int p = 0; p < PTS; ++p) {
-    if (!ok[p]) continue;
-    const int iz = z0 + p;
-    const int c = ix + g.sx * iy + g.sxy * iz;
-    R v1 = b1[p], va = ba[p], v2 = b2[p];
-    if constexpr (MODE == 1) {
-      v1 = to_flux(v1, J1, ix, iy, iz, g.dbm);
-      va = to_flux(va, JA, ix, iy, iz, g.dbm);
-      v2 = to_flux(v2, J2, ix, iy, iz, g.dbm);
-    }
-    // second flux ranges (xremap.f90:141-157; yremap.f90:142-158)
-    bool r2a = true, r2b = true;
-    if (A == 0) {
-      r2a = ix >= 1 && ix <= g.nx && iy >= 1 && iy <= g.ny && iz <= g.nz;
-      r2b = ix <= g.nx;
-    } else if (A == 1) {
-      r2b = ix >= 1 && ix <= g.nx && iy <= g.ny && iz >= 1 && iz <= g.nz;
-    }
-    if (in[p]) {
-      // first flux: b1 over 0:n+1 all, a-component over 0:n+1 all
-      v1 = v1 - f1c[p] + f1a[p];
-      R b = va + f1c[p] - f1b[p];
-      if (r2a) v2 = v2 - f2c[p] + f2a[p];
-      if (r2b) b = b + f2c[p] - f2b[p];
-      va = b;
-    }
-    if constexpr (MODE == 0) {
-      g.Bb1[c] = v1;
-      if (r2a) g.Bb2[c] = v2;
-      g.Ba[c] = va;
-    } else {
-      if constexpr (MODE == 2) {
-        v1 = from_flux(v1, J1, ix, iy, iz, g.dbm, g.rdbm);
-        va = from_flux(va, JA, ix, iy, iz, g.dbm, g.rdbm);
-        v2 = from_flux(v2, J2, ix, iy, iz, g.dbm, g.rdbm);
-      }
-      g.ob1[c] = v1;
-      g.oa[c] = va;
-      g.ob2[c] = v2;
-    }
-  }
-}
-
 // K4 + K5 + K6 for the y and z sweeps as one marching kernel.  A thread owns
 // a line along A at one (x, transverse) position of the cell box and walks a
 // chunk of it: at each point it forms the mass flux dm (K4, with the ghost
@@ -1267,13 +810,11 @@ LARE_END  // namespace lare
 
 LARE_BEGIN
 
-template <int A, class R>
 // bmode: 1 for the first sweep of a remap (B read as stored, put in flux
 // form on the way), 2 for the last (B put back from flux form), 0 between.
-void remap_sweep(Run<R>& run, bool predictor, int dt_slot, int pass[3], int bmode) {
+template <int A, class R>
+void remap_sweep(Run<R>& run, int dt_slot, int pass[3], int bmode) {
   constexpr int T1 = A == 0 ? 1 : 0, T2 = A == 2 ? 1 : 2;  // transverse axes, T1 < T2
-  constexpr int B1 = A == 0 ? 1 : 0, B2 = A == 2 ? 1 : 2;  // transported components, in file order
-  constexpr int O1 = 3 - A - B1, O2 = 3 - A - B2;          // the remaining axis for each
   const int nx = run.n[0], ny = run.n[1], nz = run.n[2];
   const int nn[3] = {nx, ny, nz};
   const int na = nn[A];
@@ -1281,10 +822,6 @@ void remap_sweep(Run<R>& run, bool predictor, int dt_slot, int pass[3], int bmod
   const int SA = A == 0 ? 1 : (A == 1 ? sx : sxy);
   const int S1 = T1 == 0 ? 1 : (T1 == 1 ? sx : sxy);
   const int S2 = T2 == 0 ? 1 : (T2 == 1 ? sx : sxy);
-  const int SB1 = B1 == 0 ? 1 : (B1 == 1 ? sx : sxy);
-  const int SB2 = B2 == 0 ? 1 : (B2 == 1 ? sx : sxy);
-  const int SO1 = O1 == 0 ? 1 : (O1 == 1 ? sx : sxy);
-  const int SO2 = O2 == 0 ? 1 : (O2 == 1 ? sx : sxy);
   Arrays<R>& Ar = run.a;
   R* const vx1 = Ar.vx1.p;
   R* const vy1 = Ar.vy1.p;
@@ -1302,7 +839,6 @@ void remap_sweep(Run<R>& run, bool predictor, int dt_slot, int pass[3], int bmod
   const A1<R> rdba = Ar.rdb[A], rdbt1 = Ar.rdb[T1], rdbt2 = Ar.rdb[T2];
   const R pass_t1 = (R)pass[T1], pass_t2 = (R)pass[T2];
   const double* sc = run.sc;
-  const bool write_cv2 = !predictor;
 
   // ---- K1: cv1, cv2, db1, dc1 over the whole cell box -1..n+2 (z-marching for
   // every FP32 sweep, the FP64 z sweep and the exact FP64 x sweep; per cell for
@@ -1332,7 +868,6 @@ void remap_sweep(Run<R>& run, bool predictor, int dt_slot, int pass[3], int bmod
     ga.nz = nz;
     ga.sx = sx;
     ga.sxy = sxy;
-    ga.write_cv2 = write_cv2;
     dim3 blk(32, 4, 1);
     dim3 grd((nx + 4 + 31) / 32, (ny + 4 + 3) / 4, 1);
     ga.chunk = march_chunk(nz + 4, grd.x * grd.y, kGeomZ, resident_blocks<k_geom_march<A, R>>(128));
@@ -1359,10 +894,8 @@ void remap_sweep(Run<R>& run, bool predictor, int dt_slot, int pass[3], int bmod
       R term_a = div_rcp(dvv[A], dba(pp[A]), rdba(pp[A]));
       R dv = (term_t1 + term_t2 + term_a) * dt;
       cv1[c] = cv[c] * (R(1) + dv);
-      if (write_cv2) {
-        dv = (term_t1 + term_t2) * dt;
-        cv2[c] = cv[c] * (R(1) + dv);
-      }
+      dv = (term_t1 + term_t2) * dt;
+      cv2[c] = cv[c] * (R(1) + dv);
       R d0 = dba(pp[A]) + dvv[A] * dt;
       db1[c] = d0;
       // dxc1 = (dxb1(p) + dxb1(min(p+1, n+2))) / 2 (xremap.f90:107-115)
@@ -1377,120 +910,15 @@ void remap_sweep(Run<R>& run, bool predictor, int dt_slot, int pass[3], int bmod
     });
   }
 
-  // ---- K2: both constrained-transport fluxes over -1..n+1
-  R* const Bp[3] = {Ar.bx.p, Ar.by.p, Ar.bz.p};
-  R* const f1 = Ar.f1.p;
-  R* const f2 = Ar.f2.p;
+  // ---- K2: B, into the second set of arrays
   {
-    BfArgs<R> ba;
-    ba.va = va;
-    ba.b1 = Bp[B1];
-    ba.b2 = Bp[B2];
-    ba.db1 = db1;
-    ba.dc1 = dc1;
-    ba.f1 = f1;
-    ba.f2 = f2;
-    ba.sc = sc;
-    ba.dt_slot = dt_slot;
-    ba.SA = SA;
-    ba.SB1 = SB1;
-    ba.SB2 = SB2;
-    ba.SO1 = SO1;
-    ba.SO2 = SO2;
-    ba.SX = 1;
-    ba.SY = A == 1 ? sxy : sx;     // the grid's second axis: z for the y sweep, y for the z sweep
-    ba.na = na;
-    ba.n0 = nx + 3;
-    ba.n1 = (A == 1 ? nz : ny) + 3;
-    ba.dbm[0] = Ar.dxb;
-    ba.dbm[1] = Ar.dyb;
-    ba.dbm[2] = Ar.dzb;
-    ba.j1 = B1;
-    ba.j2 = B2;
-    ba.ax = A;
-    const bool pre = bmode == 1;
-    const int k = run.prof_begin(A == 0 ? "remap_sweep_bflux_x" : "remap_sweep_bflux_march", 0, 7,
-                                 (double)(nx + 3) * (ny + 3) * (nz + 3));
-    if (A != 0) {
-      dim3 blk(32, 4, 1);
-      dim3 grd((ba.n0 + 31) / 32, (ba.n1 + 3) / 4, (na + 3 + kMarch - 1) / kMarch);
-      if (sizeof(R) == 8) {  // one flux per thread in FP64 (half the registers); FP32 measured the same either way
-        dim3 grd1((ba.n0 + 31) / 32, (ba.n1 + 3) / 4, 2 * ((na + 3 + kMarch - 1) / kMarch));
-        if (pre) {
-          k_bflux_march1<R, true><<<grd1, blk, 0, run.s>>>(ba);
-        } else {
-          k_bflux_march1<R, false><<<grd1, blk, 0, run.s>>>(ba);
-        }
-      } else if (pre) {
-        k_bflux_march<R, true><<<grd, blk, 0, run.s>>>(ba);
-      } else {
-        k_bflux_march<R, false><<<grd, blk, 0, run.s>>>(ba);
-      }
-    } else {
-      dim3 blk(32, 4, 1);
-      dim3 grd((nx + 3 + kXOut - 1) / kXOut, (ny + 3 + 3) / 4, nz + 3);
-      if (pre) {
-        k_bflux_x<R, true><<<grd, blk, 0, run.s>>>(ba, sx, sxy, nx, ny);
-      } else {
-        k_bflux_x<R, false><<<grd, blk, 0, run.s>>>(ba, sx, sxy, nx, ny);
-      }
-    }
-    run.prof_end(k);
-    ++run.launches;
+    R* const in[3] = {Ar.bx.p, Ar.by.p, Ar.bz.p};
+    R* const out[3] = {Ar.bx1.p, Ar.by1.p, Ar.bz1.p};
+    bsweep<A>(run, va, in, out, dt_slot, bmode);
+    std::swap(Ar.bx.p, Ar.bx1.p);
+    std::swap(Ar.by.p, Ar.by1.p);
+    std::swap(Ar.bz.p, Ar.bz1.p);
   }
-
-  // ---- K3: the four updates, each over its file's range (the first sweep
-  // of a remap also puts B in flux form, the last puts it back)
-  {
-    R* const Ba = Bp[A];
-    R* const Bb1 = Bp[B1];
-    R* const Bb2 = Bp[B2];
-    // the predictor keeps B as B0: its first sweep writes the B0 buffers,
-    // which are then swapped in (lagran.F90:945-1062)
-    const bool keep = bmode == 1 && predictor;
-    R* const B0p[3] = {Ar.bx0.p, Ar.by0.p, Ar.bz0.p};
-    BUpdArgs<R> gu;
-    gu.f1 = f1;
-    gu.f2 = f2;
-    gu.Ba = Ba;
-    gu.Bb1 = Bb1;
-    gu.Bb2 = Bb2;
-    gu.oa = keep ? B0p[A] : Ba;
-    gu.ob1 = keep ? B0p[B1] : Bb1;
-    gu.ob2 = keep ? B0p[B2] : Bb2;
-    for (int d = 0; d < 3; ++d) {
-      gu.dbm[d] = dbm[d];
-      gu.rdbm[d] = Ar.rdb[d];
-    }
-    gu.nx = nx;
-    gu.ny = ny;
-    gu.nz = nz;
-    gu.sx = sx;
-    gu.sxy = sxy;
-    gu.SA = SA;
-    gu.SB1 = SB1;
-    gu.SB2 = SB2;
-    constexpr int kPts = sizeof(R) == 4 ? kBUpdZ32 : kBUpdZ64;
-    const int e = bmode == 0 ? 2 : 5;  // points per axis: the update box 0..n+1, or the arrays' -2..n+2
-    dim3 grd((nx + e + 31) / 32, (ny + e + 3) / 4, (nz + e + kPts - 1) / kPts);
-    // words: B (3) read and written, the two fluxes read
-    const int k = run.prof_begin("remap_sweep_bupd", 0, 8, (double)(nx + e) * (ny + e) * (nz + e));
-    if (bmode == 1) {
-      k_bupdate<A, kPts, 1, R><<<grd, dim3(32, 4, 1), 0, run.s>>>(gu);
-    } else if (bmode == 2) {
-      k_bupdate<A, kPts, 2, R><<<grd, dim3(32, 4, 1), 0, run.s>>>(gu);
-    } else {
-      k_bupdate<A, kPts, 0, R><<<grd, dim3(32, 4, 1), 0, run.s>>>(gu);
-    }
-    run.prof_end(k);
-    ++run.launches;
-    if (keep) {
-      std::swap(Ar.bx.p, Ar.bx0.p);
-      std::swap(Ar.by.p, Ar.by0.p);
-      std::swap(Ar.bz.p, Ar.bz0.p);
-    }
-  }
-  if (predictor) return;  // xremap.f90:159-162 (pass flag not reset)
 
   R* const rho = Ar.rho.p;        // rho1 of the reference from here on
   R* const rho_new = Ar.rho_alt.p;
