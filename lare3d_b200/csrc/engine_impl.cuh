@@ -200,7 +200,8 @@ class EngineT : public EngineBase {
     // kernels with more than the default 48 KiB of dynamic shared memory
     if (cudaFuncSetAttribute(k_lp4_tile<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lp4_smem_bytes<R>()) !=
             cudaSuccess ||
-        bs_attributes<R>() != cudaSuccess) {
+        bs_attributes<R>() != cudaSuccess || me_attributes<R>() != cudaSuccess ||
+        vm_attributes<R>() != cudaSuccess) {
       err = "shared memory attribute";
       return LARE_ECUDA;
     }

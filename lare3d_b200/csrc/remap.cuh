@@ -7,25 +7,21 @@
 // expression over exactly the same inputs, so the results are unchanged bit
 // for bit; what changes is where intermediates live:
 //
-//   K1 geometry   cv1, cv2, dxb1 and dxc1 (xremap.f90:57-115); dxb1 at p+e_A
-//                 is recomputed in the thread for dxc1.
-//   K2 B          both constrained-transport edge fluxes (:340-470) and the
+//   K1 B          both constrained-transport edge fluxes (:340-470) and the
 //                 four flux-difference updates (:121-157) with the geometry
-//                 they need, one kernel (remap_b.cuh) into a second set of B
-//                 arrays.
-//   K4 mass flux  dm (:474-533) over the whole cell box, with dm_x_bcs
-//                 (:899-917) folded in: a ghost element is the flux computed
-//                 at its source index (the same value the copy would bring).
-//   K5 rho, eflux new rho (:174-182) into a second buffer (old rho stays
-//                 readable as rho1) and the energy flux (:539-601).
-//   K6 energy     energy update (:187-196).
+//                 they need (remap_b.cuh), into a second set of B arrays.
+//   K2 mass,      cv1 and cv2 (:57-86), dm (:474-533) over the whole cell box
+//   energy        with dm_x_bcs (:899-917) folded in, the new rho (:174-182)
+//                 into a second buffer (old rho stays readable as rho1), the
+//                 energy flux (:539-601) and the new energy (:187-196)
+//                 (remap_me.cuh).
 //   K7 vertex     vertex rho_v, cv1, cv2, dm averages and rho_v1 (:201-290).
 //   K8 momentum   the three momentum fluxes (:605-895), each times dm, and
 //   K9 velocity   the three velocity updates (:292-329), fused into one
 //                 kernel that writes the new velocities to second buffers.
 // The face-averaged vx1 written back at :265 is only read again as
 // REAL(xpass)*(...) with xpass = 0, so it is formed in K8 and not stored.
-// The predictor's sweeps (predictor_step = .TRUE.) are K2 alone.
+// The predictor's sweeps (predictor_step = .TRUE.) are K1 alone.
 //
 // Indexing is linear: c = ix + sx*iy + sxy*iz, neighbours by constant
 // offsets, with the axis a compile-time parameter.
@@ -34,171 +30,9 @@
 #include <utility>
 
 #include "remap_b.cuh"
+#include "remap_me.cuh"
 
 LARE_BEGIN
-
-// K1 as a z-marching kernel: a thread owns an (x, y) column and walks a
-// chunk of z.  Each face average (xremap.f90:64-86) sums two values of its
-// own plane and two of the plane below in that order, so the lower pair is
-// carried from the previous step instead of reloaded, and the z face below a
-// cell is the previous step's z face above it: 12 to 15 loads per cell
-// instead of 28, the same expressions, the same results bit for bit.
-constexpr int kGeomZ = 16;  // largest chunk of z (march_chunk)
-
-template <class R>
-struct GeomArgs {
-  const R* vx1;
-  const R* vy1;
-  const R* vz1;
-  const R* cv;
-  R* cv1;
-  R* cv2;
-  R* db1;
-  R* dc1;
-  A1<R> dbm[3];
-  A1<R> rdbm[3];  // reciprocals of dbm, for div_rcp
-  R pass_t1, pass_t2;
-  const double* sc;
-  int dt_slot, nx, ny, nz, sx, sxy;
-  int chunk;
-};
-
-template <int A, class R>
-__global__ void __launch_bounds__(128) k_geom_march(GeomArgs<R> g) {
-  // distinct arrays (no output is an input): restrict lets the compiler
-  // hoist the next plane's loads above this plane's stores
-  const R* __restrict__ vx1_r = g.vx1;
-  const R* __restrict__ vy1_r = g.vy1;
-  const R* __restrict__ vz1_r = g.vz1;
-  const R* __restrict__ cv_r = g.cv;
-  R* __restrict__ cv1_r = g.cv1;
-  R* __restrict__ cv2_r = g.cv2;
-  R* __restrict__ db1_r = g.db1;
-  R* __restrict__ dc1_r = g.dc1;
-  constexpr int T1 = A == 0 ? 1 : 0, T2 = A == 2 ? 1 : 2;
-  const int ix = -1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int iy = -1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-  if (ix > g.nx + 2 || iy > g.ny + 2) return;
-  const int z0 = -1 + (int)blockIdx.z * g.chunk;
-  const int z1 = min(z0 + g.chunk - 1, g.nz + 2);
-  const int sx = g.sx, sxy = g.sxy;
-  const int nn[3] = {g.nx, g.ny, g.nz};
-  const R q4 = R(0.25);
-  const R dt = (R)g.sc[g.dt_slot];
-  const R* __restrict__ vx1 = vx1_r;
-  const R* __restrict__ vy1 = vy1_r;
-  const R* __restrict__ vz1 = vz1_r;
-  constexpr int NX = A == 0 ? 3 : 2;  // x faces: c - 1, c (, c + 1)
-  constexpr int NY = A == 1 ? 3 : 2;  // y faces: c - sx, c (, c + sx)
-  const bool ahead = (A == 0 ? ix : iy) < nn[A] + 2;  // a face beyond c along A exists (A = 0, 1)
-  int c = ix + sx * iy + sxy * (z0 - 1);
-  // carried lower pairs of the x and y faces, and the z faces
-  R xa[NX], xb[NX], ya[NY], yb[NY];
-  auto xo = [&](int k) { return k - 1; };        // x offset of x face k
-  auto yo = [&](int k) { return (k - 1) * sx; }; // y offset of y face k
-#pragma unroll
-  for (int k = 0; k < NX; ++k) {
-    const bool ok = k < 2 || ahead;
-    xa[k] = ok ? vx1[c + xo(k)] : R(0);
-    xb[k] = ok ? vx1[c + xo(k) - sx] : R(0);
-  }
-#pragma unroll
-  for (int k = 0; k < NY; ++k) {
-    const bool ok = k < 2 || ahead;
-    ya[k] = ok ? vy1[c + yo(k)] : R(0);
-    yb[k] = ok ? vy1[c + yo(k) - 1] : R(0);
-  }
-  auto vzf = [&](int q) { return (vz1[q] + vz1[q - 1] + vz1[q - sx] + vz1[q - 1 - sx]) * q4; };
-  R vz_prev = vzf(c);          // z face of plane z0 - 1
-  c += sxy;
-  R vz_cur = vzf(c);           // z face of plane z0
-  // the loads of each plane are issued one plane ahead: x and y face pairs,
-  // the next z face (its four corners) and cv
-  struct Plane {
-    R xa[NX], xb[NX], ya[NY], yb[NY], z[4], cv;
-  };
-  auto fetch = [&](int q, int iz) {
-    Plane P;
-#pragma unroll
-    for (int k = 0; k < NX; ++k) {
-      const bool ok = k < 2 || ahead;
-      P.xa[k] = ok ? vx1[q + xo(k)] : R(0);
-      P.xb[k] = ok ? vx1[q + xo(k) - sx] : R(0);
-    }
-#pragma unroll
-    for (int k = 0; k < NY; ++k) {
-      const bool ok = k < 2 || ahead;
-      P.ya[k] = ok ? vy1[q + yo(k)] : R(0);
-      P.yb[k] = ok ? vy1[q + yo(k) - 1] : R(0);
-    }
-    // the z face above this plane: read by the z sweep (vz_next) and, for
-    // the other sweeps, carried as the next plane's current z face
-    const bool zok = A == 2 ? iz < g.nz + 2 : iz < z1;
-    const int qz = q + sxy;
-    P.z[0] = zok ? vz1[qz] : R(0);
-    P.z[1] = zok ? vz1[qz - 1] : R(0);
-    P.z[2] = zok ? vz1[qz - sx] : R(0);
-    P.z[3] = zok ? vz1[qz - 1 - sx] : R(0);
-    P.cv = cv_r[q];
-    return P;
-  };
-  Plane nxt = fetch(c, z0);
-  for (int iz = z0; iz <= z1; ++iz, c += sxy) {
-    const Plane cur = nxt;
-    if (iz < z1) nxt = fetch(c + sxy, iz + 1);
-    R vxfc[NX], vyfc[NY];
-#pragma unroll
-    for (int k = 0; k < NX; ++k) {
-      const R a = cur.xa[k], b = cur.xb[k];
-      vxfc[k] = (a + b + xa[k] + xb[k]) * q4;
-      xa[k] = a;
-      xb[k] = b;
-    }
-#pragma unroll
-    for (int k = 0; k < NY; ++k) {
-      const R a = cur.ya[k], b = cur.yb[k];
-      vyfc[k] = (a + b + ya[k] + yb[k]) * q4;
-      ya[k] = a;
-      yb[k] = b;
-    }
-    const R vxb = vxfc[1], vxbm = vxfc[0];
-    const R vyb = vyfc[1], vybm = vyfc[0];
-    const R vzb = vz_cur, vzbm = vz_prev;
-    const R vz_above = (cur.z[0] + cur.z[1] + cur.z[2] + cur.z[3]) * q4;
-    R vz_next = R(0);
-    if (A == 2 && iz < g.nz + 2) vz_next = vz_above;
-    const R dvv[3] = {vxb - vxbm, vyb - vybm, vzb - vzbm};
-    const int pp[3] = {ix, iy, iz};
-    // quotients by the metrics: through their reciprocals for the z sweep;
-    // the x sweep's form (three x faces live) is faster with plain division
-    auto quot = [&](R a, int d) {
-#if LARE_FAST
-      return a * g.rdbm[d](pp[d]);
-#else
-      return A == 0 ? a / g.dbm[d](pp[d]) : div_rcp(a, g.dbm[d](pp[d]), g.rdbm[d](pp[d]));
-#endif
-    };
-    const R term_t1 = quot(g.pass_t1 * dvv[T1], T1);
-    const R term_t2 = quot(g.pass_t2 * dvv[T2], T2);
-    const R term_a = quot(dvv[A], A);
-    R dv = (term_t1 + term_t2 + term_a) * dt;
-    const R cvc = cur.cv;
-    cv1_r[c] = cvc * (R(1) + dv);
-    dv = (term_t1 + term_t2) * dt;
-    cv2_r[c] = cvc * (R(1) + dv);
-    const R d0 = g.dbm[A](pp[A]) + dvv[A] * dt;
-    db1_r[c] = d0;
-    R d1 = d0;
-    if (pp[A] < nn[A] + 2) {
-      const R f = A == 0 ? vxfc[NX - 1] : (A == 1 ? vyfc[NY - 1] : vz_next);
-      const R fa = A == 0 ? vxb : (A == 1 ? vyb : vzb);
-      d1 = g.dbm[A](pp[A] + 1) + (f - fa) * dt;
-    }
-    dc1_r[c] = R(0.5) * (d0 + d1);
-    vz_prev = vz_cur;
-    vz_cur = A == 2 ? vz_next : (iz < z1 ? vz_above : R(0));
-  }
-}
 
 // K7 as a z-marching kernel: a thread owns an (x, y) column of vertices and
 // walks a chunk of z.  The eight cells around vertex (x, y, z) are the
@@ -350,7 +184,7 @@ struct MomArgs {
   const R* rv1;
   R* fp[3];  // rke only: the fluxes before their product with dm
   A1<R> dct1, dct2;
-  const double* sc;
+  double* sc;
   int dt_slot, nx, ny, nz, na, n3, sx, sxy, SA, S3;
   int chunk;
 };
@@ -384,21 +218,30 @@ __device__ __forceinline__ void mom_flux_vals(R area, R va0, R va1, R rvc, R rvp
   const R phi = fabs(v_advect) * dt / dxbu;
   const R dmu = fabs(dmc) / area / dxbu / rhou;
 #endif
+#if LARE_FAST
+  // the slopes' factors, the widths and the 1/6 in, also shared
+  const bool up = !signbit(v_advect);
+  const R dxb6 = dxbu * (R(1) / R(6));
+  const R k0 = (R(2) - phi) * rci * dxb6, ku = (R(1) + phi) * rcu * dxb6, omd = R(1) - dmu;
+#endif
 #pragma unroll
   for (int comp = 0; comp < 3; ++comp) {
     const R fm = w[comp][0], fi = w[comp][1], fp = w[comp][2], fp2 = w[comp][3];
     const R dfm = fi - fm, dfi = fp - fi, dfp = fp2 - fp;
+#if LARE_FAST
+    const R dfu = up ? dfm : dfp;
+    const R da = k0 * fabs(dfi) + ku * fabs(dfu);
+    const R Di = signed_min(lesser(lesser(R(fabs(da)), R(fabs(dfi))), R(fabs(dfu))), dfi, dfu, v_advect);
+    const R f = (up ? fi : fp) + Di * omd;
+#else
     const R fu = fi * vad_p + fp * vad_m;
     const R dfu = dfm * vad_p + dfp * vad_m;
-#if LARE_FAST
-    R Da = (R(2) - phi) * fabs(dfi) * rci + (R(1) + phi) * fabs(dfu) * rcu;
-#else
     R Da = (R(2) - phi) * fabs(dfi) / dxci + (R(1) + phi) * fabs(dfu) / dxcu;
-#endif
     Da = Da * (R(1) / R(6));
     const R ss = R(0.5) * (copysign(R(1), dfi) + copysign(R(1), dfu));
     const R Di = sign_v * ss * fmin(fmin(fabs(Da) * dxbu, fabs(dfi)), fabs(dfu));
     const R f = fu + Di * (R(1) - dmu);
+#endif
     if constexpr (BOTH) fpre[comp] = f;
     F[comp] = f * dmc;
   }
@@ -548,262 +391,6 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 4 : 8) k_mom_march(MomAr
   }
 }
 
-// K4 + K5 + K6 for the y and z sweeps as one marching kernel.  A thread owns
-// a line along A at one (x, transverse) position of the cell box and walks a
-// chunk of it: at each point it forms the mass flux dm (K4, with the ghost
-// values of dm_[yz]_bcs taken at their source index), the new density from
-// the dm below and here (K5), the energy flux (K5) and the new energy from
-// the energy flux below and here (K6).  The fluxes of the point below are
-// carried in registers, so the energy flux never reaches memory, and the new
-// energy goes to a second buffer (swapped in after the launch) because the
-// limiter of the next chunk still reads the old values.  The same
-// expressions over the same operands as the three point kernels.
-constexpr int kMEChunk = 16;  // largest chunk (march_chunk)
-
-template <class R>
-struct MEArgs {
-  const R* va;       // velocity component along A (v1)
-  const R* rho;      // old density (rho1)
-  R* rho_new;
-  const R* energy;   // old energy
-  R* energy_new;
-  R* dm;
-  const R* cv1;
-  const R* cv2;
-  const R* db1;
-  const R* dc1;
-  A1<R> dbt1, dbt2;  // widths of the transverse axes
-  const double* sc;
-  int dt_slot;
-  int SA, S1, S2, SY;  // strides along A, T1 (= x), T2, and the thread grid's second axis (= T2)
-  int na, nt1, nt2;
-  int chunk;
-  bool per;
-};
-
-template <class R>
-__global__ void __launch_bounds__(128) k_mass_energy_march(MEArgs<R> a) {
-  const int x = (int)(blockIdx.x * blockDim.x + threadIdx.x) - 1;  // T1 = x, -1..nt1+2
-  const int t = (int)(blockIdx.y * blockDim.y + threadIdx.y) - 1;  // T2, -1..nt2+2
-  if (x > a.nt1 + 2 || t > a.nt2 + 2) return;
-  const int na = a.na, SA = a.SA, S1 = a.S1, S2 = a.S2;
-  const int ia0 = -1 + (int)blockIdx.z * a.chunk;
-  const int ia1 = min(ia0 + a.chunk - 1, na + 2);
-  const bool inside_t = x >= 0 && x <= a.nt1 + 1 && t >= 0 && t <= a.nt2 + 1;  // dm's transverse range
-  const bool line0 = x <= a.nt1 && t <= a.nt2 && x >= 0 && t >= 0;          // the energy flux's
-  const bool line1 = line0 && x >= 1 && t >= 1;                              // the updates'
-  const R dt = (R)a.sc[a.dt_slot];
-  const R area = inside_t ? a.dbt1(x) * a.dbt2(t) : R(0);
-  const R* __restrict__ rho = a.rho;
-  const R* __restrict__ en = a.energy;
-  const R* __restrict__ va = a.va;
-  const R* __restrict__ dc1 = a.dc1;
-  const R* __restrict__ db1 = a.db1;
-  // K4 at ia (cell c), from its source index
-  auto mass_flux = [&](int ia, int c) -> R {
-    if (!inside_t) return R(0);
-    int sa = ia;
-    if (a.per) {
-      if (ia == na + 1) sa = 1;
-      else if (ia == na + 2) sa = 2;
-      else if (ia == -1) sa = na - 1;
-      else if (ia == 0) sa = na;
-    } else {
-      if (ia == na + 1) sa = na;
-      else if (ia == -1) sa = 0;
-      else if (ia == na + 2) return R(0);
-    }
-    const int q = c + (sa - ia) * SA;
-    const int qm = q - SA, qp = q + SA, qp2 = q + 2 * SA;
-    const R v_advect = (va[q] + va[q - S1] + va[q - S2] + va[q - S1 - S2]) * R(0.25);
-    LimOut<R> L = limiter<R>(v_advect, rho[qm], rho[q], rho[qp], rho[qp2], dc1[q], dc1[qm], dc1[qp], db1[q],
-                             db1[qp], R(0), R(0), dt, false);
-    return (L.fu + L.Di * (R(1) - L.phi)) * v_advect * dt * area;
-  };
-  // K5's energy flux at ia (cell c), 0 <= ia <= na on line0
-  auto energy_flux = [&](int c, R dmc) -> R {
-    const int cm = c - SA, cp = c + SA, cp2 = c + 2 * SA;
-    const R v_advect = (va[c] + va[c - S1] + va[c - S2] + va[c - S1 - S2]) * R(0.25);
-    LimOut<R> L = limiter<R>(v_advect, en[cm], en[c], en[cp], en[cp2], dc1[c], dc1[cm], dc1[cp], db1[c], db1[cp],
-                             R(0), R(0), dt, false);
-    const R rhou = rho[c] * L.vad_p + rho[cp] * L.vad_m;
-#if LARE_FAST
-    const R dmu = fabs(dmc) * fast_rcp(area * L.dxbu * rhou);
-#else
-    const R dmu = fabs(dmc) / area / L.dxbu / rhou;
-#endif
-    return (L.fu + L.Di * (R(1) - dmu)) * dmc;
-  };
-  const int base = x + t * a.SY;
-  // loads along the line, clamped to the cell box (a clamped value is never
-  // used: the windows reach past n + 2 only at points whose dm is a ghost
-  // value and whose energy flux is not formed)
-  auto at = [&](int ia) { return base + min(ia, na + 2) * SA; };
-  auto vface = [&](int q) { return (va[q] + va[q - S1] + va[q - S2] + va[q - S1 - S2]) * R(0.25); };
-  // the fluxes at ia0 - 1, which the first updates of the chunk read
-  R dm_prev = R(0), ef_prev = R(0);
-  if (ia0 >= 1 && ia0 - 1 <= na) {
-    dm_prev = mass_flux(ia0 - 1, at(ia0 - 1));
-    if (line0) ef_prev = energy_flux(at(ia0 - 1), dm_prev);
-  }
-  // register windows of step ia: rho and energy at ia-1..ia+2, dc1 at
-  // ia-1..ia+1, db1 at ia..ia+1, and the point's face velocity, cv1, cv2
-  R r[4], e[4], dcw[3], dbw[2];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    r[k] = rho[at(ia0 - 1 + k)];
-    e[k] = en[at(ia0 - 1 + k)];
-  }
-#pragma unroll
-  for (int k = 0; k < 3; ++k) dcw[k] = dc1[at(ia0 - 1 + k)];
-  dbw[0] = db1[at(ia0)];
-  dbw[1] = db1[at(ia0 + 1)];
-  R vf = vface(at(ia0)), c1 = a.cv1[at(ia0)], c2 = a.cv2[at(ia0)];
-  for (int ia = ia0; ia <= ia1; ++ia) {
-    const int c = at(ia);
-    // the next step's new points, a step ahead
-    const bool more = ia < ia1;
-    R nr = R(0), ne = R(0), ndc = R(0), ndb = R(0), nvf = R(0), nc1 = R(0), nc2 = R(0);
-    if (more) {
-      nr = rho[at(ia + 3)];
-      ne = en[at(ia + 3)];
-      ndc = dc1[at(ia + 2)];
-      ndb = db1[at(ia + 2)];
-      const int cn = at(ia + 1);
-      nvf = vface(cn);
-      nc1 = a.cv1[cn];
-      nc2 = a.cv2[cn];
-    }
-    // K4 at ia: from the windows, or from the source index for a ghost value
-    R dmc = R(0);
-    if (inside_t) {
-      const bool ghost = a.per ? (ia <= 0 || ia >= na + 1) : (ia == -1 || ia >= na + 1);
-      if (!ghost) {
-        LimOut<R> L = limiter<R>(vf, r[0], r[1], r[2], r[3], dcw[1], dcw[0], dcw[2], dbw[0], dbw[1], R(0), R(0),
-                                 dt, false);
-        dmc = (L.fu + L.Di * (R(1) - L.phi)) * vf * dt * area;
-      } else {
-        dmc = mass_flux(ia, c);
-      }
-    }
-    a.dm[c] = dmc;
-    const bool in1 = line1 && ia >= 1 && ia <= na;
-    R rn = r[1];
-    if (in1) rn = qdiv(r[1] * c1 + dm_prev - dmc, c2);
-    a.rho_new[c] = rn;
-    R ef = R(0);
-    if (line0 && ia >= 0 && ia <= na) {
-      LimOut<R> L = limiter<R>(vf, e[0], e[1], e[2], e[3], dcw[1], dcw[0], dcw[2], dbw[0], dbw[1], R(0), R(0), dt,
-                               false);
-      const R rhou = r[1] * L.vad_p + r[2] * L.vad_m;
-#if LARE_FAST
-      const R dmu = fabs(dmc) * fast_rcp(area * L.dxbu * rhou);
-#else
-      const R dmu = fabs(dmc) / area / L.dxbu / rhou;
-#endif
-      ef = (L.fu + L.Di * (R(1) - dmu)) * dmc;
-    }
-    R eo = e[1];
-    if (in1) eo = qdiv(e[1] * c1 * r[1] + ef_prev - ef, c2 * rn);
-    a.energy_new[c] = eo;
-    dm_prev = dmc;
-    ef_prev = ef;
-    r[0] = r[1]; r[1] = r[2]; r[2] = r[3]; r[3] = nr;
-    e[0] = e[1]; e[1] = e[2]; e[2] = e[3]; e[3] = ne;
-    dcw[0] = dcw[1]; dcw[1] = dcw[2]; dcw[2] = ndc;
-    dbw[0] = dbw[1]; dbw[1] = ndb;
-    vf = nvf; c1 = nc1; c2 = nc2;
-  }
-}
-
-// The same for the x sweep: the lanes of a warp hold consecutive x
-// positions and take their stencil neighbours (one to the left, two to the
-// right) and the fluxes of the point to their left by shuffles.  A warp
-// spans 32 positions and writes the kMEXOut = 28 whose stencils and left
-// fluxes lie inside it; ghost values of dm (dm_x_bcs) are formed from their
-// source index by direct loads.
-constexpr int kMEXOut = 28;
-
-template <class R>
-__global__ void __launch_bounds__(128) k_mass_energy_x(MEArgs<R> a, int sx, int sxy, int nx) {
-  const int lane = (int)threadIdx.x;                               // blockDim.x == 32: one warp per row
-  const int ix = -3 + (int)blockIdx.x * kMEXOut + lane;            // lane 2 holds the first output
-  const int iy = -1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-  const int iz = -1 + (int)blockIdx.z;
-  if (iy > a.nt1 + 2) return;                                      // uniform over the warp
-  const int S1 = a.S1, S2 = a.S2;
-  const int xl = min(max(ix, -2), nx + 2);                         // in-box load position
-  const int c = xl + sx * iy + sxy * iz;
-  const bool inside_t = iy >= 0 && iy <= a.nt1 + 1 && iz >= 0 && iz <= a.nt2 + 1;
-  const bool line0 = iy >= 0 && iy <= a.nt1 && iz >= 0 && iz <= a.nt2;
-  const bool line1 = line0 && iy >= 1 && iz >= 1;
-  const R dt = (R)a.sc[a.dt_slot];
-  const R area = inside_t ? a.dbt1(iy) * a.dbt2(iz) : R(0);
-  const R* __restrict__ rho = a.rho;
-  const R* __restrict__ en = a.energy;
-  const R* __restrict__ va = a.va;
-  const R* __restrict__ dc1 = a.dc1;
-  const R* __restrict__ db1 = a.db1;
-  const R r0 = rho[c], e0 = en[c], dc = dc1[c], db = db1[c];
-  const unsigned all = 0xffffffffu;
-  const R rm = __shfl_up_sync(all, r0, 1), rp = __shfl_down_sync(all, r0, 1), rp2 = __shfl_down_sync(all, r0, 2);
-  const R em = __shfl_up_sync(all, e0, 1), ep = __shfl_down_sync(all, e0, 1), ep2 = __shfl_down_sync(all, e0, 2);
-  const R dcm = __shfl_up_sync(all, dc, 1), dcp = __shfl_down_sync(all, dc, 1);
-  const R dbp = __shfl_down_sync(all, db, 1);
-  const R v_c = (va[c] + va[c - S1] + va[c - S2] + va[c - S1 - S2]) * R(0.25);
-  const int na = a.na;
-  // K4 at ix: from the lane neighbours, or from the source index for a ghost
-  R dmc = R(0);
-  if (inside_t && lane >= 1 && lane <= 29) {
-    int sa = ix;
-    bool compute = true;
-    if (a.per) {
-      if (ix == na + 1) sa = 1;
-      else if (ix == na + 2) sa = 2;
-      else if (ix == -1) sa = na - 1;
-      else if (ix == 0) sa = na;
-    } else {
-      if (ix == na + 1) sa = na;
-      else if (ix == -1) sa = 0;
-      else if (ix == na + 2) compute = false;
-    }
-    if (compute && ix >= -1 && ix <= na + 2) {
-      if (sa == ix) {
-        LimOut<R> L = limiter<R>(v_c, rm, r0, rp, rp2, dc, dcm, dcp, db, dbp, R(0), R(0), dt, false);
-        dmc = (L.fu + L.Di * (R(1) - L.phi)) * v_c * dt * area;
-      } else {
-        const int q = c + (sa - ix), qm = q - 1, qp = q + 1, qp2 = q + 2;
-        const R v_advect = (va[q] + va[q - S1] + va[q - S2] + va[q - S1 - S2]) * R(0.25);
-        LimOut<R> L = limiter<R>(v_advect, rho[qm], rho[q], rho[qp], rho[qp2], dc1[q], dc1[qm], dc1[qp], db1[q],
-                                 db1[qp], R(0), R(0), dt, false);
-        dmc = (L.fu + L.Di * (R(1) - L.phi)) * v_advect * dt * area;
-      }
-    }
-  }
-  // K5's energy flux at ix (0 <= ix <= na on line0)
-  R ef = R(0);
-  if (line0 && ix >= 0 && ix <= na && lane >= 1 && lane <= 29) {
-    LimOut<R> L = limiter<R>(v_c, em, e0, ep, ep2, dc, dcm, dcp, db, dbp, R(0), R(0), dt, false);
-    const R rhou = r0 * L.vad_p + rp * L.vad_m;
-#if LARE_FAST
-    const R dmu = fabs(dmc) * fast_rcp(area * L.dxbu * rhou);
-#else
-    const R dmu = fabs(dmc) / area / L.dxbu / rhou;
-#endif
-    ef = (L.fu + L.Di * (R(1) - dmu)) * dmc;
-  }
-  const R dm_prev = __shfl_up_sync(all, dmc, 1), ef_prev = __shfl_up_sync(all, ef, 1);
-  if (lane < 2 || lane > 29 || ix > na + 2) return;
-  a.dm[c] = dmc;
-  const bool in1 = line1 && ix >= 1 && ix <= na;
-  R rn = r0;
-  if (in1) rn = qdiv(r0 * a.cv1[c] + dm_prev - dmc, a.cv2[c]);
-  a.rho_new[c] = rn;
-  R e = e0;
-  if (in1) e = qdiv(e0 * a.cv1[c] * r0 + ef_prev - ef, a.cv2[c] * rn);
-  a.energy_new[c] = e;
-}
-
 LARE_END  // namespace lare
 
 #include "remap_vm.cuh"
@@ -830,7 +417,6 @@ void remap_sweep(Run<R>& run, int dt_slot, int pass[3], int bmode) {
   R* const va = V1[A];
   R* const cv = Ar.cv.p;
   R* const cv1 = Ar.cv1.p;
-  R* const cv2 = Ar.cv2.p;
   R* const db1 = Ar.db1.p;
   R* const dc1 = Ar.dc1.p;
   const A1<R> dbm[3] = {Ar.dxb, Ar.dyb, Ar.dzb};
@@ -840,77 +426,7 @@ void remap_sweep(Run<R>& run, int dt_slot, int pass[3], int bmode) {
   const R pass_t1 = (R)pass[T1], pass_t2 = (R)pass[T2];
   const double* sc = run.sc;
 
-  // ---- K1: cv1, cv2, db1, dc1 over the whole cell box -1..n+2 (z-marching for
-  // every FP32 sweep, the FP64 z sweep and the exact FP64 x sweep; per cell for
-  // the other FP64 sweeps, where the marching form measured no faster)
-  if (A == 2 || sizeof(R) == 4 || (A == 0 && !LARE_FAST)) {
-    GeomArgs<R> ga;
-    ga.vx1 = vx1;
-    ga.vy1 = Ar.vy1.p;
-    ga.vz1 = vz1;
-    ga.cv = cv;
-    ga.cv1 = cv1;
-    ga.cv2 = cv2;
-    ga.db1 = db1;
-    ga.dc1 = dc1;
-    ga.dbm[0] = Ar.dxb;
-    ga.dbm[1] = Ar.dyb;
-    ga.dbm[2] = Ar.dzb;
-    ga.rdbm[0] = Ar.rdb[0];
-    ga.rdbm[1] = Ar.rdb[1];
-    ga.rdbm[2] = Ar.rdb[2];
-    ga.pass_t1 = pass_t1;
-    ga.pass_t2 = pass_t2;
-    ga.sc = sc;
-    ga.dt_slot = dt_slot;
-    ga.nx = nx;
-    ga.ny = ny;
-    ga.nz = nz;
-    ga.sx = sx;
-    ga.sxy = sxy;
-    dim3 blk(32, 4, 1);
-    dim3 grd((nx + 4 + 31) / 32, (ny + 4 + 3) / 4, 1);
-    ga.chunk = march_chunk(nz + 4, grd.x * grd.y, kGeomZ, resident_blocks<k_geom_march<A, R>>(128));
-    grd.z = (nz + 4 + ga.chunk - 1) / ga.chunk;
-    const int k = run.prof_begin("remap_sweep_geom_march", 0, 8, (double)(nx + 4) * (ny + 4) * (nz + 4));
-    k_geom_march<A, R><<<grd, blk, 0, run.s>>>(ga);
-    run.prof_end(k);
-    ++run.launches;
-  } else {
-    LARE_BOXWH(run, 0, 2, 8, -1, nx + 2, -1, ny + 2, -1, nz + 2, [=] __device__(int ix, int iy, int iz) {
-      const R dt = (R)sc[dt_slot];
-      const int c = ix + sx * iy + sxy * iz;
-      // v at the two faces normal to each axis (xremap.f90:64-86)
-      auto vxf = [&](int q) { return (vx1[q] + vx1[q - sx] + vx1[q - sxy] + vx1[q - sx - sxy]) * R(0.25); };
-      auto vyf = [&](int q) { return (vy1[q] + vy1[q - 1] + vy1[q - sxy] + vy1[q - 1 - sxy]) * R(0.25); };
-      auto vzf = [&](int q) { return (vz1[q] + vz1[q - 1] + vz1[q - sx] + vz1[q - 1 - sx]) * R(0.25); };
-      R vxb = vxf(c), vxbm = vxf(c - 1);
-      R vyb = vyf(c), vybm = vyf(c - sx);
-      R vzb = vzf(c), vzbm = vzf(c - sxy);
-      R dvv[3] = {vxb - vxbm, vyb - vybm, vzb - vzbm};
-      const int pp[3] = {ix, iy, iz};
-      R term_t1 = div_rcp(pass_t1 * dvv[T1], dbt1(pp[T1]), rdbt1(pp[T1]));
-      R term_t2 = div_rcp(pass_t2 * dvv[T2], dbt2(pp[T2]), rdbt2(pp[T2]));
-      R term_a = div_rcp(dvv[A], dba(pp[A]), rdba(pp[A]));
-      R dv = (term_t1 + term_t2 + term_a) * dt;
-      cv1[c] = cv[c] * (R(1) + dv);
-      dv = (term_t1 + term_t2) * dt;
-      cv2[c] = cv[c] * (R(1) + dv);
-      R d0 = dba(pp[A]) + dvv[A] * dt;
-      db1[c] = d0;
-      // dxc1 = (dxb1(p) + dxb1(min(p+1, n+2))) / 2 (xremap.f90:107-115)
-      R d1 = d0;
-      if (pp[A] < na + 2) {
-        const int q = c + SA;
-        R f = A == 0 ? vxf(q) : (A == 1 ? vyf(q) : vzf(q));
-        R fa = A == 0 ? vxb : (A == 1 ? vyb : vzb);
-        d1 = dba(pp[A] + 1) + (f - fa) * dt;
-      }
-      dc1[c] = R(0.5) * (d0 + d1);
-    });
-  }
-
-  // ---- K2: B, into the second set of arrays
+  // ---- K1: B, into the second set of arrays
   {
     R* const in[3] = {Ar.bx.p, Ar.by.p, Ar.bz.p};
     R* const out[3] = {Ar.bx1.p, Ar.by1.p, Ar.bz1.p};
@@ -921,55 +437,36 @@ void remap_sweep(Run<R>& run, int dt_slot, int pass[3], int bmode) {
   }
 
   R* const rho = Ar.rho.p;        // rho1 of the reference from here on
-  R* const rho_new = Ar.rho_alt.p;
-  R* const energy = Ar.energy.p;
   R* const dm = Ar.dm.p;
-  R* const eflux = Ar.flux.p;
-  const bool per = run.p.per[A];
-  const int nt1 = nn[T1], nt2 = nn[T2];
-
+  const int swept = 3 - pass[0] - pass[1] - pass[2];
+  const R* const cv2 = swept == 2 ? Ar.cv.p : Ar.cv2.p;  // the third sweep ends at the grid itself
   {
-    // ---- K4 + K5 + K6 in one kernel (marching along A for the y and z
-    // sweeps, warp shuffles along x for the x sweep); the new energy is
-    // swapped in
     MEArgs<R> me;
-    me.va = va;
-    me.rho = rho;
-    me.rho_new = rho_new;
-    me.energy = energy;
-    me.energy_new = eflux;  // the energy-flux array is free in this form
-    me.dm = dm;
-    me.cv1 = cv1;
-    me.cv2 = cv2;
-    me.db1 = db1;
-    me.dc1 = dc1;
-    me.dbt1 = dbt1;
-    me.dbt2 = dbt2;
-    me.sc = sc;
-    me.dt_slot = dt_slot;
-    me.SA = SA;
-    me.S1 = S1;
-    me.S2 = S2;
-    me.SY = S2;
-    me.na = na;
-    me.nt1 = nt1;
-    me.nt2 = nt2;
-    me.per = per;
-    dim3 blk(32, 4, 1);
-    // words: rho, energy, va, dc1, db1, cv1, cv2 read; dm, rho_new, energy written
-    const int k = run.prof_begin(A == 0 ? "remap_sweep_mass_energy_x" : "remap_sweep_mass_energy_march", 0, 10,
-                                 (double)(nx + 4) * (ny + 4) * (nz + 4));
-    if (A == 0) {
-      dim3 grd((nx + 4 + kMEXOut - 1) / kMEXOut, (ny + 4 + 3) / 4, nz + 4);
-      k_mass_energy_x<R><<<grd, blk, 0, run.s>>>(me, sx, sxy, nx);
-    } else {
-      dim3 grd((nt1 + 4 + 31) / 32, (nt2 + 4 + 3) / 4, 1);
-      me.chunk = march_chunk(na + 4, grd.x * grd.y, kMEChunk, resident_blocks<k_mass_energy_march<R>>(128));
-      grd.z = (na + 4 + me.chunk - 1) / me.chunk;
-      k_mass_energy_march<R><<<grd, blk, 0, run.s>>>(me);
+    for (int d = 0; d < 3; ++d) {
+      me.v[d] = V1[d];
+      me.m[d] = dbm[d];
+      me.r[d] = Ar.rdb[d];
+      me.pass[d] = pass[d];
     }
-    run.prof_end(k);
-    ++run.launches;
+    me.rho = rho;
+    me.rho_new = Ar.rho_alt.p;
+    me.energy = Ar.energy.p;
+    me.energy_new = Ar.flux.p;  // swapped in below
+    me.dm = dm;
+    me.cv = Ar.cv.p;
+    me.cv1 = cv1;
+    me.cv2 = Ar.cv2.p;
+    me.db1 = run.p.rke ? db1 : nullptr;
+    me.dc1 = dc1;
+    me.sc = run.sc;
+    me.dt_slot = dt_slot;
+    me.nx = nx;
+    me.ny = ny;
+    me.nz = nz;
+    me.sx = sx;
+    me.sxy = sxy;
+    me.per = run.p.per[A];
+    mass_energy_sweep<A>(run, me, swept);
     std::swap(Ar.energy.p, Ar.flux.p);
   }
 
@@ -1033,7 +530,7 @@ void remap_sweep(Run<R>& run, int dt_slot, int pass[3], int bmode) {
     gm.rv1 = rv1;
     gm.dct1 = dct1;
     gm.dct2 = dct2;
-    gm.sc = sc;
+    gm.sc = run.sc;
     gm.dt_slot = dt_slot;
     gm.nx = nx;
     gm.ny = ny;
@@ -1046,26 +543,19 @@ void remap_sweep(Run<R>& run, int dt_slot, int pass[3], int bmode) {
     gm.S3 = A == 1 ? sxy : sx;
     const bool rke = run.p.rke != 0;
     for (int q = 0; q < 3; ++q) gm.fp[q] = rke ? Ar.rke_f[q].p : nullptr;
-    // words: fused, v (3), v1, db1, dc1, rho, cv1, cv2, dm read and the new v (3) written
+    // words: fused, v (3), v1, rho, cv1, cv2, dm read and the new v (3) written
     const char* site = fused_vm ? (A == 0 ? "remap_sweep_vert_mom_x" : "remap_sweep_vert_mom_march")
                                 : (A == 0 ? "remap_sweep_mom_x" : "remap_sweep_mom_march");
-    const int k = run.prof_begin(site, 0, fused_vm ? 13 : (rke ? 17 : 14), (double)(nx + 1) * (ny + 1) * (nz + 1));
+    const int k = run.prof_begin(site, 0, fused_vm ? 11 : (rke ? 17 : 14), (double)(nx + 1) * (ny + 1) * (nz + 1));
     if (fused_vm) {
       VMArgs<R> vm;
       vm.m = gm;
+      vm.dba = dbm[A];
       vm.rho = rho;
       vm.cv1 = cv1;
       vm.cv2 = cv2;
       vm.dm = dm;
-      if constexpr (A == 0) {
-        dim3 grd((nx + 1 + kVMXOut - 1) / kVMXOut, (ny + 1 + 3) / 4, nz + 1);
-        k_vm_x<R><<<grd, dim3(32, 4, 1), 0, run.s>>>(vm);
-      } else {
-        dim3 grd((nx + 1 + 31) / 32, (gm.n3 + 1 + 3) / 4, 1);
-        vm.m.chunk = march_chunk(na + 1, grd.x * grd.y, kMomA, resident_blocks<k_vm_march<A, R>>(128));
-        grd.z = (na + 1 + vm.m.chunk - 1) / vm.m.chunk;
-        k_vm_march<A, R><<<grd, dim3(32, 4, 1), 0, run.s>>>(vm);
-      }
+      vm_launch<A>(run, vm);
     } else if (A == 0) {
       dim3 grd((nx + 1 + 30) / 31, (ny + 1 + 3) / 4, nz + 1);
       if (rke)

@@ -60,6 +60,40 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
+// A ring of NS shared-memory slots filled by one thread and read by all warps
+// of a block: a full barrier a slot counts the bytes of its copies, an empty
+// one the warps that are done with it.  Step k uses slot k % NS.  A wait that
+// runs out (a copy that never arrives) raises LARE_ECUDA in sc and is not
+// repeated, so that the block still ends.
+template <int NS>
+struct TileRing {
+  uint32_t full, empty, base;  // shared-memory addresses: barriers, slot 0
+  int bytes;                   // a slot
+  double* sc;
+  bool dead = false;
+  // one thread, before a block barrier
+  __device__ __forceinline__ void init(int warps) {
+    for (int s = 0; s < NS; ++s) {
+      mbar_init(full + 8 * s, 1);
+      mbar_init(empty + 8 * s, warps);
+    }
+    mbar_init_fence();
+  }
+  __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity) {
+    if (!dead && !mbar_wait(bar, parity)) {
+      dead = true;
+      sc[SC_ERROR] = (double)LARE_ECUDA;
+    }
+  }
+  __device__ __forceinline__ void wait_full(int slot, uint32_t parity) { wait(full + 8 * slot, parity); }
+  // a warp is done with a slot
+  __device__ __forceinline__ void release(int slot) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0)
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty + 8 * slot) : "memory");
+  }
+};
+
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
 // against the driver library).
 inline PFN_cuTensorMapEncodeTiled_v12000 tma_encoder() {
