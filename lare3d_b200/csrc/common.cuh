@@ -175,7 +175,12 @@ enum Slot {
 };
 // Integer min-reduction targets (bit patterns of positive doubles order
 // like unsigned integers).
-enum USlot { U_DTMIN = 0, U_DTRMIN, U_DTPARAB, U_NSLOTS = 4 };
+// U_DONE: finished blocks of the sum in flight.  Each is left reset by the
+// kernel that reads it.
+enum USlot { U_DTMIN = 0, U_DTRMIN, U_DTPARAB, U_DONE, U_NSLOTS = 4 };
+
+// The bits of DBL_MAX: no minimum yet.
+constexpr unsigned long long kMinReset = 0x7fefffffffffffffull;
 
 struct Box {
   int lo[3], hi[3];
@@ -248,8 +253,8 @@ inline void launch_scalar(cudaStream_t s, long long& count, Fn fn) {
 
 // ---------------------------------------------------------------------
 // Deterministic sums: each block reduces NV values per thread in a fixed
-// tree and writes its partials; one block then adds the partials in a
-// fixed order.  Results are run-to-run reproducible (not equal to a
+// tree and writes its partials; the last block then adds them in a fixed
+// order.  Results are run-to-run reproducible (not equal to a
 // serial left-to-right sum, which no parallel order can reproduce).
 template <int NV>
 __device__ __forceinline__ void block_sum_write(double (&v)[NV], double* partial, int bid) {
@@ -274,15 +279,46 @@ __device__ __forceinline__ void block_sum_write(double (&v)[NV], double* partial
   }
 }
 
-// Each block covers `planes` consecutive planes (kSumPlanes by default:
-// fewer partials for the final pass; 1 for heavy point functions, whose
-// planes would otherwise run one after another); a thread adds its points
-// plane by plane, so the order of every sum is fixed.
+// Each block covers `planes` consecutive planes (at least kSumPlanes: fewer
+// partials for the final sum); a thread adds its points plane by plane, so the
+// order of every sum is fixed.
 constexpr int kSumPlanes = 4;
+
+// The partials of all blocks added in a fixed order (1024 strided sums, then
+// two warp trees) by the block that finishes last: a sum is one launch.
+// `done` counts the finished blocks and is left at zero.
+template <int NV>
+__device__ __forceinline__ void last_block_sum(const double* partial, int nb, double* out, int accumulate,
+                                               unsigned* done) {
+  __shared__ bool last;
+  __shared__ double sh[NV][32];
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x, nt = blockDim.x * blockDim.y;
+  __threadfence();
+  __syncthreads();  // this block's partials are written
+  if (tid == 0) last = atomicAdd(done, 1u) == (unsigned)nb - 1u;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int t = tid; t < 1024; t += nt)
+    for (int q = 0; q < NV; ++q) {
+      double x = 0.0;
+      for (int b = t; b < nb; b += 1024) x += __ldcg(partial + (size_t)b * NV + q);
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if ((t & 31) == 0) sh[q][t >> 5] = x;
+    }
+  __syncthreads();
+  if (tid < 32)
+    for (int q = 0; q < NV; ++q) {
+      double x = sh[q][tid];
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if (tid == 0) out[q] = accumulate ? out[q] + x : x;
+    }
+  if (tid == 0) *done = 0u;
+}
 
 template <int NV, class Fn>
 __global__ void __launch_bounds__(256) k_box_sum(int i0, int j0, int k0, int ni, int nj, int nk, int planes, Fn fn,
-                                                 double* partial) {
+                                                 double* partial, double* out, int accumulate, unsigned* done) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   int j = blockIdx.y * blockDim.y + threadIdx.y;
   double v[NV];
@@ -298,26 +334,7 @@ __global__ void __launch_bounds__(256) k_box_sum(int i0, int j0, int k0, int ni,
   }
   int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
   block_sum_write<NV>(v, partial, bid);
-}
-
-template <int NV>
-__global__ void __launch_bounds__(1024) k_sum_partials(const double* partial, int nb, double* out, int accumulate) {
-  __shared__ double sh[NV][32];
-  int t = threadIdx.x;
-  for (int q = 0; q < NV; ++q) {
-    double x = 0.0;
-    for (int b = t; b < nb; b += blockDim.x) x += partial[(size_t)b * NV + q];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if ((t & 31) == 0) sh[q][t >> 5] = x;
-  }
-  __syncthreads();
-  if (t < 32) {
-    for (int q = 0; q < NV; ++q) {
-      double x = sh[q][t];
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      if (t == 0) out[q] = accumulate ? out[q] + x : x;
-    }
-  }
+  last_block_sum<NV>(partial, (int)(gridDim.x * gridDim.y * gridDim.z), out, accumulate, done);
 }
 
 // Min of positive doubles through their bit patterns.

@@ -306,19 +306,23 @@ inline void ghost(Run<R>& run, const GSpec& g, A3<R> a, A3<R>* b = nullptr, A3<R
 
 // Deterministic sum of NV values over a box, into sc[slot..] (+=).
 // site names the launch in the profile; words: the algorithmic words per
-// point the kernel moves.
+// point the kernel moves.  Planes per block: few enough blocks (4096) that
+// the last one adds their partials in a few microseconds, which at 256^3 took
+// 35 us for the 21,000 blocks of 4 planes.
 template <int NV, class R, class Fn>
 inline void box_sum(Run<R>& run, const char* site, int i0, int i1, int j0, int j1, int k0, int k1, Fn fn, int slot,
-                    bool acc, int words = 0, int planes = kSumPlanes) {
+                    bool acc, int words = 0) {
   int ni = i1 - i0 + 1, nj = j1 - j0 + 1, nk = k1 - k0 + 1;
   dim3 blk(64, 4, 1);
-  dim3 grd((ni + 63) / 64, (nj + 3) / 4, (nk + planes - 1) / planes);
-  int nb = grd.x * grd.y * grd.z;
+  dim3 grd((ni + 63) / 64, (nj + 3) / 4, 1);
+  int planes = kSumPlanes;
+  while (planes < 32 && (long long)grd.x * grd.y * ((nk + planes - 1) / planes) > 4096) planes *= 2;
+  grd.z = (nk + planes - 1) / planes;
   int k = run.prof_begin(site, 0, words, (double)ni * nj * nk);
-  k_box_sum<NV><<<grd, blk, 0, run.s>>>(i0, j0, k0, ni, nj, nk, planes, fn, run.partial);
-  k_sum_partials<NV><<<1, 1024, 0, run.s>>>(run.partial, nb, run.sc + slot, acc ? 1 : 0);
+  k_box_sum<NV><<<grd, blk, 0, run.s>>>(i0, j0, k0, ni, nj, nk, planes, fn, run.partial, run.sc + slot, acc ? 1 : 0,
+                                        (unsigned*)(run.us + U_DONE));
   run.prof_end(k);
-  run.launches += 2;
+  ++run.launches;
 }
 
 template <int NV, class R, class Fn>
@@ -400,10 +404,22 @@ template <class R> inline void boundary_conditions(Run<R>& r) {
   b.add(r.g_node, r.a.vx.p, r.a.vy.p, r.a.vz.p);
   ghost_flush(r, b);
 }
-// energy_bcs + density_bcs at the end of lagrangian_step (lagran.F90:196-197)
+// energy_bcs + density_bcs at the end of lagrangian_step (lagran.F90:196-197),
+// with the velocity_bcs after the corrector's new velocity (:409): nothing in
+// between reads the velocity's ghosts unless a side is open.
 template <class R> inline void end_of_step_bcs(Run<R>& r) {
   GhostBatch<R> b;
   b.add(r.g_cell, r.a.energy.p, r.a.rho.p);
+  if (!r.any_open) b.add(r.g_node, r.a.vx.p, r.a.vy.p, r.a.vz.p);
+  ghost_flush(r, b);
+}
+// bfield_bcs + energy_bcs at the end of a resistive sub-cycle
+template <class R> inline void resistive_bcs(Run<R>& r) {
+  GhostBatch<R> b;
+  b.add(r.g_bx, r.a.bx.p);
+  b.add(r.g_by, r.a.by.p);
+  b.add(r.g_bz, r.a.bz.p);
+  b.add(r.g_cell, r.a.energy.p);
   ghost_flush(r, b);
 }
 
@@ -530,7 +546,6 @@ void calc_s_stages(Run<R>& run, int dt_slot) {
     larsen(ix, iy, iz) = q_fs / sqrt(q_fs2 + q_sp2);
   });
   unsigned long long* us = run.us;
-  launch_scalar(run.s, run.launches, [=] __device__() { us[U_DTPARAB] = (unsigned long long)__double_as_longlong(1.e10); });
   box_min<1>(run, "parabolic_dt_min", 1, nx, 1, ny, 1, nz, [=] __device__(int ix, int iy, int iz, double* v) {
     R kappa1 = k0 * larsen(ix, iy, iz);
     const R x = pip ? xia(ix, iy, iz) : xi;
@@ -547,6 +562,7 @@ void calc_s_stages(Run<R>& run, int dt_slot) {
   const bool f32 = sizeof(R) == 4;
   launch_scalar(run.s, run.launches, [=] __device__() {
     double dtp_min = __longlong_as_double((long long)us[U_DTPARAB]);
+    us[U_DTPARAB] = kMinReset;
     double dt = sc[dt_slot];
     double stages, dt_parab;
     if (f32) {
@@ -843,7 +859,8 @@ void eulerian_remap(Run<R>& run, int step) {
       default: remap_sweep<2>(run, SC_DT, pass, bmode); break;
     }
   }
-  bfield_bcs(run);
+  // (the last sweep's boundary_conditions already filled the converted B:
+  // bfield_bcs at remap.f90:128 would write the same values again)
 }
 
 // Pull the scalar slots to the host (one sync).
@@ -854,44 +871,109 @@ cudaError_t pull_scalars(Run<R>& run) {
 }
 
 // ---------------------------------------------------------------------
-// diagnostics.F90:517-609 energy_account into sc[SC_EN_B..SC_EN_INT].
+// diagnostics.F90:517-609 energy_account into sc[SC_EN_B..SC_EN_INT], in one
+// pass over the vertices 0:n, the cells among them.  A thread walks `planes`
+// planes of its column and carries the lower quad of the vertex' eight cells
+// (mass and volume): 17 loads a point instead of 30,
+// 0.27 against 0.38 ms at 256^3 (FP64) for the two point kernels it replaces.
+template <class R>
+struct EnergyArgs {
+  const R *bx, *by, *bz, *cv, *energy, *rho, *vx, *vy, *vz;
+  double *partial, *out;
+  unsigned* done;
+  int nx, ny, nz, sx, sxy, planes;
+};
+
+template <class R>
+__global__ void __launch_bounds__(256) k_energy_account(EnergyArgs<R> g) {
+  const int ix = (int)(blockIdx.x * blockDim.x + threadIdx.x), iy = (int)(blockIdx.y * blockDim.y + threadIdx.y);
+  const int z0 = (int)blockIdx.z * g.planes, z1 = min(z0 + g.planes - 1, g.nz);
+  double v[3] = {0.0, 0.0, 0.0};
+  if (ix <= g.nx && iy <= g.ny) {
+    const int sx = g.sx;
+    int c = ix + sx * iy + g.sxy * z0;
+    // a plane's quad around the vertex: its sums, and the cell itself
+    struct Quad {
+      double r, w, r0, w0;
+    };
+    auto quad = [&](int q, double r, double w) {  // added to the sums r and w
+      const int o[4] = {0, 1, sx, 1 + sx};
+      Quad t{r, w, 0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const double cw = g.cv[q + o[k]], rw = (double)g.rho[q + o[k]] * cw;
+        t.r += rw;
+        t.w += cw;
+        if (k == 0) {
+          t.r0 = rw;
+          t.w0 = cw;
+        }
+      }
+      return t;
+    };
+    auto both = [&](int q, double r, double w, Quad& own) {  // a quad alone, and added to the sums below it
+      const int o[4] = {0, 1, sx, 1 + sx};
+      Quad t{r, w, 0.0, 0.0};
+      own = Quad{0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const double cw = g.cv[q + o[k]], rw = (double)g.rho[q + o[k]] * cw;
+        t.r += rw;
+        t.w += cw;
+        own.r = k == 0 ? rw : own.r + rw;
+        own.w = k == 0 ? cw : own.w + cw;
+        if (k == 0) {
+          own.r0 = rw;
+          own.w0 = cw;
+        }
+      }
+      return t;
+    };
+    Quad lo = quad(c, 0.0, 0.0);
+    double dlo = z0 >= 1 ? (double)g.bz[c - g.sxy] : 0.0;
+    const double ex = ix == 0 || ix == g.nx ? 0.5 : 1.0, ey = iy == 0 || iy == g.ny ? 0.5 : 1.0;
+    for (int iz = z0; iz <= z1; ++iz, c += g.sxy) {
+      Quad up;
+      const Quad t = both(c + g.sxy, lo.r, lo.w, up);
+      const double d0 = g.bz[c];
+      if (ix >= 1 && iy >= 1 && iz >= 1) {
+        const double b0 = g.bx[c], b1 = g.bx[c - 1], c0 = g.by[c], c1 = g.by[c - sx];
+        double w1 = (b0 * b0 + b1 * b1) * 0.5;
+        const double w2 = (c0 * c0 + c1 * c1) * 0.5, w3 = (d0 * d0 + dlo * dlo) * 0.5;
+        w1 = (w1 + w2 + w3) * 0.5;
+        v[0] += w1 * lo.w0;
+        v[2] += (double)g.energy[c] * lo.r0;
+      }
+      const double ux = g.vx[c], uy = g.vy[c], uz = g.vz[c];
+      // rho_v cv_v = (sum rho cv / sum cv) (sum cv / 8)
+      double w1 = t.r / t.w * (t.w * 0.125) * (ux * ux + uy * uy + uz * uz);
+      w1 = w1 * ex * ey;
+      if (iz == 0 || iz == g.nz) w1 = w1 * 0.5;
+      v[1] += w1 * 0.5;
+      lo = up;
+      dlo = d0;
+    }
+  }
+  const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+  block_sum_write<3>(v, g.partial, bid);
+  last_block_sum<3>(g.partial, (int)(gridDim.x * gridDim.y * gridDim.z), g.out, 0, g.done);
+}
+
 template <class R>
 void energy_account(Run<R>& run) {
   const int nx = run.n[0], ny = run.n[1], nz = run.n[2];
   Arrays<R>& A = run.a;
-  auto bx = A.bx, by = A.by, bz = A.bz, cv = A.cv, energy = A.energy, rho = A.rho;
-  auto vx = A.vx, vy = A.vy, vz = A.vz;
-  box_sum<2>(run, "energy_account_cells", 1, nx, 1, ny, 1, nz, [=] __device__(int ix, int iy, int iz, double* v) {
-    int ixm = ix - 1, iym = iy - 1, izm = iz - 1;
-    double b0 = bx(ix, iy, iz), b1 = bx(ixm, iy, iz), c0 = by(ix, iy, iz), c1 = by(ix, iym, iz);
-    double d0 = bz(ix, iy, iz), d1 = bz(ix, iy, izm);
-    double w1 = (b0 * b0 + b1 * b1) * 0.5;
-    double w2 = (c0 * c0 + c1 * c1) * 0.5;
-    double w3 = (d0 * d0 + d1 * d1) * 0.5;
-    w1 = (w1 + w2 + w3) * 0.5;
-    v[0] = w1 * (double)cv(ix, iy, iz);
-    v[1] = (double)energy(ix, iy, iz) * (double)rho(ix, iy, iz) * (double)cv(ix, iy, iz);
-  }, SC_EN_B, false);
-  // SC_EN_B and SC_EN_B+1 hold en_b and en_int; move en_int to its slot.
-  double* sc = run.sc;
-  launch_scalar(run.s, run.launches, [=] __device__() { sc[SC_EN_INT] = sc[SC_EN_B + 1]; });
-  box_sum<1>(run, "energy_account_vertices", 0, nx, 0, ny, 0, nz, [=] __device__(int ix, int iy, int iz, double* v) {
-    int ixp = ix + 1, iyp = iy + 1, izp = iz + 1;
-    auto r = [&](int a, int b, int c) { return (double)rho(a, b, c) * (double)cv(a, b, c); };
-    auto w = [&](int a, int b, int c) { return (double)cv(a, b, c); };
-    double rv = r(ix, iy, iz) + r(ixp, iy, iz) + r(ix, iyp, iz) + r(ixp, iyp, iz) + r(ix, iy, izp) + r(ixp, iy, izp) +
-                r(ix, iyp, izp) + r(ixp, iyp, izp);
-    double cvv = w(ix, iy, iz) + w(ixp, iy, iz) + w(ix, iyp, iz) + w(ixp, iyp, iz) + w(ix, iy, izp) + w(ixp, iy, izp) +
-                 w(ix, iyp, izp) + w(ixp, iyp, izp);
-    rv = rv / cvv;
-    cvv = cvv * 0.125;
-    double ux = vx(ix, iy, iz), uy = vy(ix, iy, iz), uz = vz(ix, iy, iz);
-    double w1 = rv * cvv * (ux * ux + uy * uy + uz * uz);
-    if (ix == 0 || ix == nx) w1 = w1 * 0.5;
-    if (iy == 0 || iy == ny) w1 = w1 * 0.5;
-    if (iz == 0 || iz == nz) w1 = w1 * 0.5;
-    v[0] = w1 * 0.5;
-  }, SC_EN_KE, false);
+  dim3 grd((nx + 1 + 63) / 64, (ny + 1 + 3) / 4, 1);
+  int planes = march_chunk(nz + 1, grd.x * grd.y, 32, resident_blocks<k_energy_account<R>>(256));
+  // few enough partials for the last block (box_sum), and room for them
+  while (planes < 64 && (long long)grd.x * grd.y * ((nz + planes) / planes) > 4096) planes *= 2;
+  grd.z = (nz + planes) / planes;
+  const EnergyArgs<R> g{A.bx.p,      A.by.p, A.bz.p, A.cv.p, A.energy.p, A.rho.p, A.vx.p, A.vy.p, A.vz.p, run.partial,
+                        run.sc + SC_EN_B, (unsigned*)(run.us + U_DONE), nx, ny, nz, run.sx, run.sxy, planes};
+  const int k = run.prof_begin("energy_account", 0, 9, (double)(nx + 1) * (ny + 1) * (nz + 1));
+  k_energy_account<R><<<grd, dim3(64, 4, 1), 0, run.s>>>(g);
+  run.prof_end(k);
+  ++run.launches;
 }
 
 LARE_END  // namespace lare

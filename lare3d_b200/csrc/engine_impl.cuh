@@ -252,6 +252,13 @@ class EngineT : public EngineBase {
     dflag = dalloc<int>(1, err);
     if (!run.sc || !run.us || !run.partial || !staging || !dflag) return LARE_ENOMEM;
     cudaMemsetAsync(run.sc, 0, SC_NSLOTS * sizeof(double), run.s);
+    {
+      unsigned long long* us = run.us;  // as each reader leaves them
+      launch_scalar(run.s, run.launches, [=] __device__() {
+        us[U_DTMIN] = us[U_DTRMIN] = us[U_DTPARAB] = kMinReset;
+        us[U_DONE] = 0ull;
+      });
+    }
     if (cudaMallocHost(&run.host_sc, SC_NSLOTS * sizeof(double)) != cudaSuccess) { err = "pinned"; return LARE_ENOMEM; }
 
     // 1-D metrics: dxb(-1:n+2), dxc(-1:n+1) per axis, grav(-1:nz+2).

@@ -284,7 +284,6 @@ void resistive_update(Run<R>& run) {
       carry_outside(run, nb[q], ob[q], lo, hi, a, b);
     }
   }
-  bfield_bcs(run);
   // RS3: ohmic heating (1:n), MAX(energy, 0) (-1:n+2) and the
   // total_ohmic_heating sum over vertices 0:n (:1270-1328)
   R* const energy = A.energy.p;
@@ -321,7 +320,7 @@ void resistive_update(Run<R>& run) {
       v[0] = (double)w1;
     }
   }, SC_OHM_TOT, true, ctb ? 8 : 6);
-  energy_bcs(run);
+  resistive_bcs(run);  // RS3 reads no B, so its fill waits for the energy's
 }
 
 // ---------------------------------------------------------------------
@@ -477,9 +476,15 @@ void set_dt(Run<R>& run) {
     run.set_dt_first = false;
     if (run.p.restart) {
       const double d = run.p.dt_from_restart;
+      const bool resist = run.p.resistive_mhd != 0;
       launch_scalar(run.s, run.launches, [=] __device__() {
         sc[SC_DT] = d;
         sc[SC_DT2] = 0.5 * d;
+        if (resist) {
+          const int n = (int)(d / sc[SC_DTR]) + 1;
+          sc[SC_SUBSTEPS] = (double)n;
+          sc[SC_DTSUB] = d / (double)n;
+        }
       });
       return;
     }
@@ -507,10 +512,6 @@ void set_dt(Run<R>& run) {
     });
     run.gamma_boris_one = !boris;
   }
-  launch_scalar(run.s, run.launches, [=] __device__() {
-    us[U_DTMIN] = (unsigned long long)__double_as_longlong(DBL_MAX);
-    us[U_DTRMIN] = (unsigned long long)__double_as_longlong(DBL_MAX);
-  });
   box_min<2>(run, "set_dt_min", 0, nx, 0, ny, 0, nz, [=] __device__(int ix, int iy, int iz, double* v) {
     const int c = ix + sx * iy + sxy * iz;
     R w1 = bx[c] * bx[c] + by[c] * by[c] + bz[c] * bz[c];
@@ -542,32 +543,48 @@ void set_dt(Run<R>& run) {
   }, U_DTMIN, cowling ? 11 : (resistive ? 10 : 9));
   const double mult = run.p.dt_multiplier;
   const bool f32 = sizeof(R) == 4;
-  launch_scalar(run.s, run.launches, [=] __device__() {
+  const bool cond = run.p.conduction != 0;
+  const bool subcycles = resistive && !run.capturing;  // a recorded step's loop counts them itself
+  auto minima = [=] __device__() {
     double dtm = __longlong_as_double((long long)us[U_DTMIN]);
     double dtrm = __longlong_as_double((long long)us[U_DTRMIN]);
+    us[U_DTMIN] = us[U_DTRMIN] = kMinReset;
     if (f32) {
       dtm = fmin(dtm, (double)FLT_MAX);
       dtrm = fmin(dtrm, (double)FLT_MAX);
     }
     sc[SC_DT] = mult * dtm;
     sc[SC_DTR] = mult * dtrm;
-  });
-  if (run.p.conduction) {
-    calc_s_stages(run, SC_DT);
+  };
+  auto clock = [=] __device__() {
+    const double dt = sc[SC_DT];
+    sc[SC_TIME] = sc[SC_TIME] + dt;
+    sc[SC_DT2] = 0.5 * dt;
+    if (subcycles) {  // lagran.F90:139-143
+      const int n = (int)(dt / sc[SC_DTR]) + 1;
+      sc[SC_SUBSTEPS] = (double)n;
+      sc[SC_DTSUB] = dt / (double)n;
+    }
+  };
+  if (!cond) {
     launch_scalar(run.s, run.launches, [=] __device__() {
-      const double ss_limit = 60;
-      int ns = (int)sc[SC_STAGES];
-      if (ns >= ss_limit) {
-        double f1 = 2.0 * ss_limit * ss_limit - 9.0;
-        double f2 = (double)(2 * ns * ns - 9);
-        sc[SC_DT] = sc[SC_DT] * f1 / f2;
-        sc[SC_DTR] = sc[SC_DTR] * f1 / f2;
-      }
+      minima();
+      clock();
     });
+    return;
   }
+  launch_scalar(run.s, run.launches, [=] __device__() { minima(); });
+  calc_s_stages(run, SC_DT);
   launch_scalar(run.s, run.launches, [=] __device__() {
-    sc[SC_TIME] = sc[SC_TIME] + sc[SC_DT];
-    sc[SC_DT2] = 0.5 * sc[SC_DT];
+    const double ss_limit = 60;
+    int ns = (int)sc[SC_STAGES];
+    if (ns >= ss_limit) {
+      double f1 = 2.0 * ss_limit * ss_limit - 9.0;
+      double f2 = (double)(2 * ns * ns - 9);
+      sc[SC_DT] = sc[SC_DT] * f1 / f2;
+      sc[SC_DTR] = sc[SC_DTR] * f1 / f2;
+    }
+    clock();
   });
 }
 
@@ -902,7 +919,7 @@ void predictor_corrector_step(Run<R>& run) {
     R* const ov[3] = {A.qx.p, A.qy.p, A.qz.p};
     carry_velocity(run, nv, ov);
   }
-  velocity_bcs(run);
+  if (run.any_open) velocity_bcs(run);  // else with end_of_step_bcs
   open_bcs(run);  // lagran.F90:410-412 (no launch unless a side is open)
   // PC4 (1:n): final cv1, energy, visc_dep, rho; total_visc_heating
   R* const cv1w = A.cv1.p;
@@ -1051,12 +1068,6 @@ int lagrangian_step(Run<R>& run, int step) {
     int rc = resistive_subcycles_captured(run);
     if (rc) return rc;
   } else if (run.p.resistive_mhd) {
-    launch_scalar(run.s, run.launches, [=] __device__() {
-      double dt = sc[SC_DT];
-      int substeps = (int)(dt / sc[SC_DTR]) + 1;
-      sc[SC_SUBSTEPS] = (double)substeps;
-      sc[SC_DTSUB] = dt / (double)substeps;
-    });
     if (pull_scalars(run) != cudaSuccess) return LARE_ECUDA;
     int substeps = (int)run.host_sc[SC_SUBSTEPS];
     double dtv = run.host_sc[SC_DT];
