@@ -72,11 +72,36 @@ NeutralPar neutral_par(const Run<R>& run) {
   return NeutralPar{p.gamma, p.ionise_pot, p.f_bar, p.t_bar, p.r_bar, p.tr, p.eta_bar};
 }
 
+// get_neutral with its derivative in t (dbof/dt = -bof (1/(2t) + 3 t_bar /
+// (4 t^2)) from the two factors above), for the root search below: the value
+// is a few rounding errors off get_neutral's own.
+__device__ __forceinline__ double neutral_slope(double t_v, double rho_v, const NeutralPar& q, double& slope) {
+  const double bof = 1.0 / (0.5 * q.f_bar * q.tr * sqrt(t_v)) *
+                     cw_exp((0.25 * (t_v / q.tr - 1.0) + 1.0) * q.t_bar / t_v);
+  const double rt = 1.0 / t_v, qb = q.r_bar * rho_v * bof, s = sqrt(1.0 + qb);
+  const double r = 0.5 * (s - 1.0), ri = 1.0 / (1.0 + r);
+  slope = -0.25 * qb * (0.5 + 0.75 * q.t_bar * rt) * rt / s * (ri * ri);
+  return r * ri;
+}
+
 // neutral.f90:158-195 neutral_fraction on the energy-like array e (the
 // energy itself, or an RKL2 stage that conduct.f90:402-404 has just copied
 // into it).  A cell whose bracket [(gamma-1) max((e-chi)/2, tiny),
 // (gamma-1) e] is empty raises LARE_EEOS, where the reference prints
 // 'Temperature bounds problem' and stops.
+//
+// The reference bisects on fa(x) = x - (gamma-1)(e - (1-xi(x)) chi)/(2-xi(x)),
+// about 27 evaluations to |dx| < 1e-8 or |fa| < 1e-8, and its xi is that of
+// its last midpoint.  The same midpoints are visited here, but fa is evaluated
+// only at the few whose sign or size is not already known: xi falls with x
+// (its exponent and 1/sqrt(t) do), so fa' >= 1 and |x - root| <= |fa(x)|.  A
+// Newton search (four or five evaluations) gives an x with |fa| < 1e-8 and
+// with it a bracket of the root; at a midpoint further than kSure from that
+// bracket fa has the bracket's side's sign and more than 1e-8 in size, which
+// is all that the bisection uses.  kSure is thousands of times fa's rounding
+// error (a few ulp of x, which is of order 1 to 1e3 in normalised units), so
+// the branches taken, the last midpoint and xi are the reference's bit for
+// bit.  Bound by the FP64 pipe: 0.092 against 0.173 ms on 84^3 cells.
 template <class R>
 void neutral_fraction(Run<R>& run, A3<R> e) {
   const int nx = run.n[0], ny = run.n[1], nz = run.n[2];
@@ -92,16 +117,61 @@ void neutral_fraction(Run<R>& run, A3<R> e) {
       sc[SC_ERROR] = (double)LARE_EEOS;
       return;
     }
+    // a bracket [lo, hi] of the root, from the evaluated points
+    double lo = ta1, hi = ta2;
+    if (rho0 >= 0.0) {  // (a negative density reverses the balance's slope)
+      double x = 0.5 * (ta1 + ta2);
+      for (int it = 0; it < 8; ++it) {
+        double ds;
+        const double xa = neutral_slope(x, rho0, q, ds);
+        const double d = 1.0 / (2.0 - xa), h = g1 * (e0 - (1.0 - xa) * ip) * d;
+        const double f = x - h;
+        if (!(fabs(f) < DBL_MAX)) break;  // (also NaN: the plain bisection below)
+        // f' >= 1: the root lies within |f| of x, on the other side
+        if (f > 0.0) {
+          hi = fmin(hi, x);
+          lo = fmax(lo, x - f);
+        } else {
+          lo = fmax(lo, x);
+          hi = fmin(hi, x - f);
+        }
+        if (fabs(f) < 1.e-8) break;
+        const double step = f / (1.0 - g1 * ip * d * ds - h * d * ds);
+        const double y = x - step;
+        x = y > lo && y < hi ? y : 0.5 * (lo + hi);
+      }
+    }
+    const double kSure = fmax(2.e-8, 1.e-12 * ta2);
+    lo -= kSure;
+    hi += kSure;
+    // below this the balance's exponent passes 300 and fa may overflow: evaluated
+    const double room = 300.0 - 0.25 * q.t_bar / q.tr;
+    const double cold = room > 0.0 ? 0.75 * q.t_bar / room : ta2;
+    // the midpoints; the lanes of a warp walk to their next one to evaluate
+    // and evaluate together
     double dx = ta2 - ta1, t = ta1, x = ta1, xi_a = 0.0;
-    for (int loop = 1; loop <= 100; ++loop) {
-      dx = dx / 2.0;
-      x = t + dx;
-      xi_a = get_neutral(x, rho0, q);
-      const double fa = x - g1 * (e0 - (1.0 - xi_a) * ip) / (2.0 - xi_a);
-      if (fa <= 0.0) t = x;
-      if (fabs(dx) < 1.e-8 || fabs(fa) < 1.e-8) break;
+    bool known = false;  // xi_a is x's
+    for (int loop = 0;;) {
+      known = false;
+      bool end = false;
+      while (!end && !known) {
+        ++loop;
+        dx = dx / 2.0;
+        x = t + dx;
+        known = (x >= lo && x <= hi) || x <= cold;
+        end = fabs(dx) < 1.e-8 || loop == 100;
+        if (!known && x < lo) t = x;
+      }
+      if (known) {
+        xi_a = get_neutral(x, rho0, q);
+        const double fa = x - g1 * (e0 - (1.0 - xi_a) * ip) / (2.0 - xi_a);
+        if (fa <= 0.0) t = x;
+        end = end || fabs(fa) < 1.e-8;
+      }
+      if (end) break;
     }
     // neutral.f90:191 recomputes get_neutral(x, rho0): the same value
+    if (!known) xi_a = get_neutral(x, rho0, q);
     xi(ix, iy, iz) = (R)xi_a;
   });
 }
