@@ -18,21 +18,16 @@
 // regrouped (and T^{5/2} = T^2 sqrt(T)), agrees with the reference to
 // rounding (relative 1e-12 in FP64).
 //
-// Stage kernel: a CTA owns a 32 x 8 column of cells and walks up a chunk of
-// z, holding the temperature of planes z-1, z, z+1 (one-cell x/y halo) in
-// shared memory, the x and y face fluxes of the current plane in shared
-// memory and the z face flux below each cell in a register carried to the
-// next plane, so each face flux is formed once.  A cell adds its six scaled
-// face fluxes in the order in which the reference's scatter delivers them:
+// Stage kernel: each face flux is formed once; a cell adds its six scaled face
+// fluxes in the order in which the reference's scatter delivers them:
 //   +Fz(c-ez), +Fy(c-ey), +Fx(c-ex), -Fx(c), -Fy(c), -Fz(c).
 #pragma once
 
+#include "tma.cuh"
+
 LARE_BEGIN
 
-constexpr int kCTX = 32, kCTY = 8, kCZ = 16;  // CTA tile (x, y) and z chunk
-constexpr int kCW = kCTX + 2;                 // plane row length with halo
-constexpr int kCPlane = kCW * (kCTY + 2);
-
+constexpr int kCTY = 8, kCZ = 32;             // rows of a CTA tile, largest chunk of z (march_chunk)
 // Coefficients of every face of cells 0..n (conduct.f90:170-275 regrouped).
 template <class R>
 void face_coefficients(Run<R>& run) {
@@ -90,11 +85,18 @@ void face_coefficients(Run<R>& run) {
 
 template <class R>
 struct StageArgs {
-  TempOf<R> T;                      // temperature of the stage input
-  A3<R> k[9];                       // face coefficients
-  A3<R> y2, y1, y0, lc0, rho, out;  // stage arrays
+  R* lc0;                           // Lc_Y0: written by stage 1
+  R* out;
+  const R* kz[3];                   // the z faces' coefficients
+  const R* y2;                      // the stage input where the temperature is an array of its own, else null
+  double* sc;
+  R tc, te0;                        // temperature of the input: tc * (y - te0)
   R k0, mt, mu, nu, omn, gt;
-  int dt_slot, nx, ny, nz;
+  int dt_slot, nx, ny, nz, sx, sxy;
+  int chunk;
+};
+struct StageMaps {
+  CUtensorMap T, k[9], rho, y0, y1, lc0;
 };
 
 template <class R>
@@ -110,166 +112,213 @@ __device__ __forceinline__ R face_q(R k0, R T0, R T1, R kn, R k1, R s1, R k2, R 
 // face to lane 30 (the high face of every cell comes from the lane above by
 // a shuffle, so no lane forms a face twice).  Each thread also forms the y
 // face flux on the low side of its cell into shared memory, where the row
-// above reads it as its high face; the top row forms its high face itself.
-// The z face flux on the high side is carried to the next plane.  The
-// temperature of planes z-1, z, z+1 with a one-cell x/y halo sits in shared
-// memory, loaded a plane ahead.
+// below reads it as its high face; the top row forms its high face itself.
+// The z face flux on the high side is carried to the next plane.
+//
+// The planes arrive by TMA two steps ahead: the stage input with a one-cell x/y
+// halo in a ring of four slots, of which three are read, and the nine face
+// coefficients, rho, Y0, Y1 and Lc_Y0 of the plane itself in a ring of two.
+// The input becomes the temperature in place a step before it is read (its
+// value at the thread's own cell stays in a register).  One barrier a step
+// orders that, the y faces and the reuse of slots.  With each array loaded by each thread a plane
+// ahead a stage took 0.30 ms at 256^3 in FP32 and 0.136 ms on 160 x 129 x 177
+// in FP64 (400 and 530 instructions a point, 118 registers in FP64); now 0.20
+// and 0.116 ms.  Its floor is 15 words, 0.155 and 0.067 ms; bound by
+// instruction issue and, in FP64, by 16 warps an SM.  (Rings of six and three
+// slots left one CTA an SM in FP64: 0.183 ms.)
 constexpr int kSTX = 31;  // cells per tile along x (a warp of 32 lanes)
-constexpr int kSW = kSTX + 2;
-constexpr int kSPlane = kSW * (kCTY + 2);
-
+constexpr int kStT = 4, kStD = 2;  // slots of the two rings
 template <class R>
-struct StagePre {
-  R kx[3], ky[3], ky2[3], kz[3];
-  R rho, y0, y1, y2, lc;
+struct StageTile {
+  static constexpr int W = sizeof(R) == 8 ? 36 : 40;  // 34 elements from the aligned start
+  static constexpr int t = (W * (kCTY + 2) * (int)sizeof(R) + 127) / 128 * 128;
+  static constexpr int h = (W * (kCTY + 1) * (int)sizeof(R) + 127) / 128 * 128;  // y coefficients: a row below
+  static constexpr int c = (W * kCTY * (int)sizeof(R) + 127) / 128 * 128;
+  static constexpr int kx = 0, kz = 3 * c, rho = 6 * c, y0 = 7 * c, y1 = 8 * c, lc = 9 * c, ky = 10 * c;
+  static constexpr int slot = 10 * c + 3 * h;
+  static constexpr unsigned sent_t = W * sizeof(R) * (kCTY + 2);
+  static constexpr unsigned sent = W * sizeof(R) * (10 * kCTY + 3 * (kCTY + 1));
+  static constexpr unsigned sent1 = sent - W * sizeof(R) * 2 * kCTY;             // stage 1: no Y1, no Lc_Y0
+  static constexpr size_t smem = 128 + (size_t)kStT * t + (size_t)kStD * slot;
 };
 
-// FIRST: stage 1 (y2 = energy = Y0): Lc_Y0 = flux / rho and
+// FIRST: stage 1 (Y0 the input): Lc_Y0 = flux / rho and
 //        out = Y0 + mt * dt * Lc_Y0.
 // else:  stage j: out = mu Y2 + nu Y1 + (1 - mu - nu) Y0 + mt dt Lc + gt dt Lc_Y0
 //        with Lc the flux of T(Y2) / rho.
 template <class R, bool FIRST>
-__global__ void __launch_bounds__(32 * kCTY, sizeof(R) == 4 ? 4 : 2)
-    k_rkl2_stage(StageArgs<R> a, const double* __restrict__ sc) {
-  __shared__ R Ts[3][kSPlane];
-  __shared__ R fy[kCTY + 1][32];
+__global__ void __launch_bounds__(32 * kCTY, sizeof(R) == 4 ? 5 : 2)
+    k_rkl2_stage(const __grid_constant__ StageMaps maps, StageArgs<R> a) {
+  using L = StageTile<R>;
+  extern __shared__ unsigned char st_smem[];
+  __shared__ R fy[2][kCTY + 1][32];
+  __shared__ __align__(8) unsigned long long bars[kStT];
+  constexpr int W = L::W;
   const int nx = a.nx, ny = a.ny, nz = a.nz;
   const int lane = threadIdx.x, ty = threadIdx.y;
-  const int tid = ty * 32 + lane;
-  const int ix0 = 1 + blockIdx.x * kSTX, iy0 = 1 + blockIdx.y * kCTY;
-  const int iz0 = 1 + blockIdx.z * kCZ;
-  const int iz1 = min(nz, iz0 + kCZ - 1);
+  const int ix0 = 1 + (int)blockIdx.x * kSTX, iy0 = 1 + (int)blockIdx.y * kCTY;
+  const int iz0 = 1 + (int)blockIdx.z * a.chunk;
+  const int iz1 = min(nz, iz0 + a.chunk - 1);
   const int ix = ix0 + lane, iy = iy0 + ty;
-  // lane 31 only forms the x face below its cell (the high x face of lane 30)
-  const bool own = lane < kSTX;
-  const bool active = own && ix <= nx && iy <= ny;            // cells this tile updates
-  const bool hx = ix - 1 <= nx && iy <= ny;                   // x face at ix - 1 (low side)
-  const bool hy = own && ix <= nx && iy - 1 <= ny;            // y face at iy - 1 (low side)
+  const bool active = lane < kSTX && ix <= nx && iy <= ny;    // cells this tile updates
   const bool top = ty == kCTY - 1;                            // the top row also forms its high y face
-  const bool hy2 = own && top && ix <= nx && iy <= ny;
-  const bool cell = active;                                   // z faces of the cells updated here
-  const int sx = a.T.y.sx, sxy = a.T.y.sxy;
-  const int cxy = min(ix, nx + 2) + sx * min(iy, ny + 2);     // this thread's column (clamped)
-  // the (up to two) plane elements this thread loads, as column offsets
-  int off[2];
-  bool has[2];
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const int e = tid + q * 32 * kCTY;
-    has[q] = e < kSPlane;
-    const int jj = has[q] ? e / kSW : 0, ii = has[q] ? e - jj * kSW : 0;
-    off[q] = min(ix0 - 1 + ii, nx + 2) + sx * min(iy0 - 1 + jj, ny + 2);
-  }
-  const R tc = a.T.c, te0 = a.T.e0;
-  const R* __restrict__ ysrc = a.T.y.p;
-  const R dt = (R)sc[a.dt_slot];
-  auto load_plane = [&](int k) {
-    R* d = Ts[(k + 3) % 3];
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-      if (has[q]) d[tid + q * 32 * kCTY] = tc * (ysrc[off[q] + sxy * k] - te0);
-  };
-  auto fetch = [&](int k) {
-    StagePre<R> q;
-    const int c = cxy + sxy * k;
+  unsigned char* const buf = st_smem + ((128u - (smem_addr(st_smem) & 127u)) & 127u);
+  unsigned char* const dat = buf + kStT * L::t;
+  const uint32_t buf_s = smem_addr(buf), dat_s = buf_s + kStT * L::t, bar_s = smem_addr(bars);
+  const int e0 = ix0 + 1, ea = e0 & ~(kTmaAlign<R> - 1);      // element of ix0 - 1, counted from x = -2
+  // step s: the input's plane iz0 + s + 1 and the other arrays' plane iz0 + s;
+  // steps -2 and -1 bring the input's planes iz0 - 1 and iz0
+  auto issue = [&](int s) {
+    const int q = s + 2, p = iz0 + s + 2;
+    const uint32_t bar = bar_s + 8 * (q % kStT);
+    mbar_expect(bar, s < 0 ? L::sent_t : L::sent_t + (FIRST ? L::sent1 : L::sent));
+    tma_load_3d(buf_s + (q % kStT) * L::t, &maps.T, ea, iy0 + 1, p + 1, bar);
+    if (s < 0) return;
+    const uint32_t d = dat_s + (s % kStD) * L::slot;
+    const int r = iy0 + 2;
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-      q.kx[m] = hx ? a.k[m].p[c - 1] : R(0);
-      q.ky[m] = hy ? a.k[3 + m].p[c - sx] : R(0);
-      q.ky2[m] = hy2 ? a.k[3 + m].p[c] : R(0);
-      q.kz[m] = cell ? a.k[6 + m].p[c] : R(0);
+      tma_load_3d(d + L::kx + m * L::c, &maps.k[m], ea, r, p, bar);
+      tma_load_3d(d + L::ky + m * L::h, &maps.k[3 + m], ea, r - 1, p, bar);
+      tma_load_3d(d + L::kz + m * L::c, &maps.k[6 + m], ea, r, p, bar);
     }
-    q.rho = active ? a.rho.p[c] : R(1);
-    q.y0 = active ? a.y0.p[c] : R(0);
-    q.y1 = (active && !FIRST) ? a.y1.p[c] : R(0);
-    q.y2 = (active && !FIRST) ? a.y2.p[c] : R(0);
-    q.lc = (active && !FIRST) ? a.lc0.p[c] : R(0);
-    return q;
+    tma_load_3d(d + L::rho, &maps.rho, ea, r, p, bar);
+    tma_load_3d(d + L::y0, &maps.y0, ea, r, p, bar);
+    if (!FIRST) {
+      tma_load_3d(d + L::y1, &maps.y1, ea, r, p, bar);
+      tma_load_3d(d + L::lc, &maps.lc0, ea, r, p, bar);
+    }
   };
-  // z face above cell e of plane slots pm (lower) and pp (upper)
-  auto zface = [&](const R* pm, const R* pp, int e, R k6, R k7, R k8) {
-    return face_q(a.k0, pm[e], pp[e], k6, k7, (pp[e + 1] + pm[e + 1]) - (pp[e - 1] + pm[e - 1]), k8,
-                  (pp[e + kSW] + pm[e + kSW]) - (pp[e - kSW] + pm[e - kSW]));
-  };
-  // y face between cell e - kSW and cell e of plane slots Pm, P0, Pp
-  auto yface = [&](const R* Pm, const R* P0, const R* Pp, int e, const R (&k)[3]) {
-    const int b = e - kSW;
-    return face_q(a.k0, P0[b], P0[e], k[0], k[1], (P0[b + 1] + P0[e + 1]) - (P0[b - 1] + P0[e - 1]), k[2],
-                  (Pp[b] + Pp[e]) - (Pm[b] + Pm[e]));
-  };
-  const int ec = (ty + 1) * kSW + lane + 1;  // this thread's cell in a plane slot
-  load_plane(iz0 - 1);
-  load_plane(iz0);
-  R fz_m = R(0);
-  R b6 = R(0), b7 = R(0), b8 = R(0);
-  if (cell) {
-    const int c = cxy + sxy * (iz0 - 1);
-    b6 = a.k[6].p[c];
-    b7 = a.k[7].p[c];
-    b8 = a.k[8].p[c];
+  const int steps = iz1 - iz0 + 1;
+  const bool boss = lane == 0 && ty == 0;
+  if (boss) {
+    for (int q = 0; q < kStT; ++q) mbar_init(bar_s + 8 * q, 1);
+    mbar_init_fence();
+    for (int s = -2; s < 2 && s < steps; ++s) issue(s);
   }
-  __syncthreads();
-  if (cell) fz_m = zface(Ts[(iz0 + 2) % 3], Ts[iz0 % 3], ec, b6, b7, b8);
-  StagePre<R> nxt = fetch(iz0);
-  for (int iz = iz0; iz <= iz1; ++iz) {
-    const StagePre<R> cur = nxt;
-    load_plane(iz + 1);
-    if (iz < iz1) nxt = fetch(iz + 1);
-    __syncthreads();
-    const R* Pm = Ts[(iz + 2) % 3];
-    const R* P0 = Ts[iz % 3];
-    const R* Pp = Ts[(iz + 1) % 3];
-    R fx_lo = R(0);
-    if (hx) {
-      const int e = ec - 1;  // face between cells ix - 1 and ix
-      fx_lo = face_q(a.k0, P0[e], P0[e + 1], cur.kx[0], cur.kx[1],
-                     (P0[e + kSW + 1] + P0[e + kSW]) - (P0[e - kSW + 1] + P0[e - kSW]), cur.kx[2],
-                     (Pp[e + 1] + Pp[e]) - (Pm[e + 1] + Pm[e]));
+  bool dead = false;  // a copy never arrived: flagged, and no more waiting
+  auto await = [&](int s) {
+    const int q = s + 2;
+    if (!dead && !mbar_wait(bar_s + 8 * (q % kStT), (uint32_t)(q / kStT) & 1u)) {
+      dead = true;
+      a.sc[SC_ERROR] = (double)LARE_ECUDA;
     }
+  };
+  const R tc = a.tc, te0 = a.te0, k0 = a.k0;
+  const R dt = (R)a.sc[a.dt_slot];
+  // this thread's cell in a plane of the input and in the other tiles, and the
+  // halo element that it turns into a temperature (84 of them)
+  const int ec = (ty + 1) * W + (e0 - ea) + lane + 1, cc = ty * W + (e0 - ea) + lane + 1;
+  const int tid = ty * 32 + lane;
+  const int eh = (e0 - ea) + (tid < 68 ? (tid < 34 ? tid : (kCTY + 1) * W + tid - 34)
+                                       : ((tid - 68) / 2 + 1) * W + (tid & 1) * 33);
+  auto plane = [&](int s) { return reinterpret_cast<R*>(buf + ((s + 2) % kStT) * L::t); };
+  auto convert = [&](int s) {
+    await(s);
+    R* const p = plane(s);
+    const R own = p[ec];
+    p[ec] = tc * (own - te0);
+    if (tid < 84) p[eh] = tc * (p[eh] - te0);
+    return own;
+  };
+  // z face above the cell of planes lo (lower) and hi
+  auto zface = [&](const R* lo, const R* hi, R k6, R k7, R k8) {
+    return face_q(k0, lo[0], hi[0], k6, k7, (hi[1] + lo[1]) - (hi[-1] + lo[-1]), k8,
+                  (hi[W] + lo[W]) - (hi[-W] + lo[-W]));
+  };
+  // y face between the cells at e - W and e of planes Pm, P0, Pp
+  auto yface = [&](const R* Pm, const R* P0, const R* Pp, R k3, R k4, R k5) {
+    return face_q(k0, P0[-W], P0[0], k3, k4, (P0[-W + 1] + P0[1]) - (P0[-W - 1] + P0[-1]), k5,
+                  (Pp[-W] + Pp[0]) - (Pm[-W] + Pm[0]));
+  };
+  __syncthreads();  // the barriers are set up
+  convert(-2);
+  R own0 = convert(-1), own1 = convert(0);  // the input at this cell, planes iz and iz + 1
+  __syncthreads();
+  R fz_m = R(0);
+  {
+    // the z face below the chunk
+    const int c = min(ix, nx + 2) + a.sx * min(iy, ny + 2) + a.sxy * (iz0 - 1);
+    fz_m = zface(plane(-2) + ec, plane(-1) + ec, a.kz[0][c], a.kz[1][c], a.kz[2][c]);
+  }
+  for (int s = 0; s < steps; ++s) {
+    const R* const Pm = plane(s - 2) + ec;
+    const R* const P0 = plane(s - 1) + ec;
+    const R* const Pp = plane(s) + ec;
+    const unsigned char* const sl = dat + (s % kStD) * L::slot;
+    auto at = [&](int off) { return reinterpret_cast<const R*>(sl + off)[cc]; };
+    // x face between cells ix - 1 and ix
+    const R* const kx = reinterpret_cast<const R*>(sl + L::kx) + cc - 1;
+    const R fx_lo = face_q(k0, P0[-1], P0[0], kx[0], kx[L::c / (int)sizeof(R)],
+                           (P0[W] + P0[W - 1]) - (P0[-W] + P0[-W - 1]), kx[2 * L::c / (int)sizeof(R)],
+                           (Pp[0] + Pp[-1]) - (Pm[0] + Pm[-1]));
     const R fx_hi = __shfl_down_sync(0xffffffffu, fx_lo, 1);
-    if (hy) fy[ty][lane] = yface(Pm, P0, Pp, ec, cur.ky);
-    if (hy2) fy[kCTY][lane] = yface(Pm, P0, Pp, ec + kSW, cur.ky2);
-    R fz_p = R(0);
-    if (cell) fz_p = zface(P0, Pp, ec, cur.kz[0], cur.kz[1], cur.kz[2]);
+    // (the y coefficients' tile starts a row lower, so cc is the row below)
+    const R* const ky = reinterpret_cast<const R*>(sl + L::ky) + cc;
+    R(*const f)[32] = fy[s & 1];
+    f[ty][lane] = yface(Pm, P0, Pp, ky[0], ky[L::h / (int)sizeof(R)], ky[2 * L::h / (int)sizeof(R)]);
+    if (top)
+      f[kCTY][lane] = yface(Pm + W, P0 + W, Pp + W, ky[W], ky[W + L::h / (int)sizeof(R)],
+                            ky[W + 2 * L::h / (int)sizeof(R)]);
+    const R fz_p = zface(P0, Pp, at(L::kz), at(L::kz + L::c), at(L::kz + 2 * L::c));
+    const R rr = R(1) / at(L::rho), v0 = at(L::y0);
+    const R v1 = FIRST ? R(0) : at(L::y1), l0 = FIRST ? R(0) : at(L::lc), v2 = own0;
+    own0 = own1;
+    if (s + 1 < steps) own1 = convert(s + 1);
     __syncthreads();
+    // every thread is past the last step: its slots are free
+    if (boss && s + 2 < steps) {
+      // the copy overwrites a plane that threads wrote (converted) before the barrier
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      issue(s + 2);
+    }
     if (active) {
-      R f = R(0);
-      f = f + fz_m;
-      f = f + fy[ty][lane];
-      f = f + fx_lo;
-      f = f - fx_hi;
-      f = f - fy[ty + 1][lane];
-      f = f - fz_p;
-      const int c = cxy + sxy * iz;
+      R g = fz_m;
+      g = g + f[ty][lane];
+      g = g + fx_lo;
+      g = g - fx_hi;
+      g = g - f[ty + 1][lane];
+      g = g - fz_p;
+      const int c = ix + a.sx * iy + a.sxy * (iz0 + s);
+      const R Lc = rr * g;
       if (FIRST) {
-        const R lc = (R(1) / cur.rho) * f;
-        a.lc0.p[c] = lc;
-        a.out.p[c] = cur.y0 + a.mt * dt * lc;
+        a.lc0[c] = Lc;
+        a.out[c] = v0 + a.mt * dt * Lc;
       } else {
-        const R c0 = a.gt * dt * cur.lc;
-        const R Lc = (R(1) / cur.rho) * f;
+        const R c0 = a.gt * dt * l0;
         const R c1 = a.mt * dt * Lc;
-        const R v = a.mu * cur.y2 + a.nu * cur.y1 + a.omn * cur.y0;
-        a.out.p[c] = v + c1 + c0;
+        const R v = a.mu * (a.y2 ? a.y2[c] : v2) + a.nu * v1 + a.omn * v0;
+        a.out[c] = v + c1 + c0;
       }
     }
     fz_m = fz_p;
   }
 }
 
+// Dynamic shared memory beyond the default 48 KiB, once per context.
+template <class R>
+inline cudaError_t stage_attributes() {
+  cudaError_t e = cudaFuncSetAttribute(k_rkl2_stage<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)StageTile<R>::smem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_rkl2_stage<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)StageTile<R>::smem);
+  return e;
+}
+
 template <class R, bool FIRST>
 void rkl2_stage(Run<R>& run, int line, const TempOf<R>& T, A3<R> y2, A3<R> y1, A3<R> y0, A3<R> out, int dt_slot,
                 R mt, R mu, R nu, R omn, R gt) {
+  using L = StageTile<R>;
   const int nx = run.n[0], ny = run.n[1], nz = run.n[2];
   StageArgs<R> a;
-  a.T = T;
-  for (int q = 0; q < 9; ++q) a.k[q] = run.a.kf[q];
-  a.y2 = y2;
-  a.y1 = y1;
-  a.y0 = y0;
-  a.lc0 = run.a.Lc_Y0;
-  a.rho = run.a.rho;
-  a.out = out;
+  a.lc0 = run.a.Lc_Y0.p;
+  a.out = out.p;
+  for (int q = 0; q < 3; ++q) a.kz[q] = run.a.kf[6 + q].p;
+  a.y2 = T.y.p == y2.p ? nullptr : y2.p;
+  a.sc = run.sc;
+  a.tc = T.c;
+  a.te0 = T.e0;
   a.k0 = (R)run.p.kappa_0;
   a.mt = mt;
   a.mu = mu;
@@ -280,10 +329,25 @@ void rkl2_stage(Run<R>& run, int line, const TempOf<R>& T, A3<R> y2, A3<R> y1, A
   a.nx = nx;
   a.ny = ny;
   a.nz = nz;
-  dim3 grid((nx + kSTX - 1) / kSTX, (ny + kCTY - 1) / kCTY, (nz + kCZ - 1) / kCZ);
+  a.sx = run.sx;
+  a.sxy = run.sxy;
+  StageMaps maps;
+  const long long f = 2 + 2LL * run.sx + 2LL * run.sxy;
+  const auto map = [&](CUtensorMap* m, const A3<R>& x, int rows) {
+    if (!tma_map(m, (const R*)x.p - f, run.n, run.sx, run.sxy, L::W, rows, 1)) run.launch_error = true;
+  };
+  map(&maps.T, T.y, kCTY + 2);
+  for (int q = 0; q < 9; ++q) map(&maps.k[q], run.a.kf[q], q / 3 == 1 ? kCTY + 1 : kCTY);
+  map(&maps.rho, run.a.rho, kCTY);
+  map(&maps.y0, y0, kCTY);
+  map(&maps.y1, y1, kCTY);
+  map(&maps.lc0, run.a.Lc_Y0, kCTY);
+  dim3 grid((nx + kSTX - 1) / kSTX, (ny + kCTY - 1) / kCTY, 1);
+  a.chunk = march_chunk(nz, grid.x * grid.y, kCZ, resident_blocks<k_rkl2_stage<R, FIRST>>(32 * kCTY, L::smem));
+  grid.z = (nz + a.chunk - 1) / a.chunk;
   // words per point: T stencil input, 9 coefficients, rho, Lc_Y0, output (+ Y1, Y0 after stage 1)
   const int k = run.prof_begin("rkl2_stage", line, FIRST ? 13 : 15, (double)nx * ny * nz);
-  k_rkl2_stage<R, FIRST><<<grid, dim3(32, kCTY, 1), 0, run.s>>>(a, run.sc);
+  k_rkl2_stage<R, FIRST><<<grid, dim3(32, kCTY, 1), L::smem, run.s>>>(maps, a);
   run.prof_end(k);
   ++run.launches;
 }

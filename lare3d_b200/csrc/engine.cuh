@@ -438,20 +438,26 @@ inline int resident_blocks(int threads, size_t smem = 0) {
 }
 // Points of a marched axis of length len that one block of a marching kernel
 // walks, for a launch of `tiles` blocks across it, `resident` of which fit on
-// the GPU at once.  A chunk loads its stencil again, so longer is cheaper: cap
-// where that still makes two full waves, else as long as one wave allows (a
-// second, partial one would cost as much as the first), down to 4 on small
-// grids, where the march's latency is the kernel's time.  With fixed chunks of
-// 16 and 32 a 64^3 grid left most SMs idle: the march of eta_calc took 52 us
-// on 96 x 80 x 121 with 8 % of the resident blocks launched.
+// the GPU at once: the number of chunks that makes the fewest steps, a wave of
+// blocks taking a chunk's points and about kMarchStart steps to fill its
+// windows.  So a large grid gets long chunks (up to cap), a small one as many
+// as run at once, down to 4 points, and no last wave is left nearly empty.
+// With fixed chunks of 16 and 32 a 64^3 grid left most SMs idle (the march of
+// eta_calc took 52 us on 96 x 80 x 121 with 8 % of the resident blocks).
+constexpr int kMarchStart = 4;
 inline int march_chunk(int len, int tiles, int cap, int resident) {
-  int n = (len + cap - 1) / cap;
-  if ((long long)tiles * n < 2LL * resident) {
-    n = resident / tiles;
-    if (n < 1) n = 1;
-    if (n > (len + 3) / 4) n = (len + 3) / 4;
+  const int n0 = (len + cap - 1) / cap, n1 = (len + 3) / 4;
+  int best = n0;
+  long long least = LLONG_MAX;
+  for (int n = n0; n <= n1; ++n) {
+    const long long waves = ((long long)tiles * n + resident - 1) / resident;
+    const long long steps = waves * ((len + n - 1) / n + kMarchStart);
+    if (steps < least) {
+      least = steps;
+      best = n;
+    }
   }
-  return (len + n - 1) / n;
+  return (len + best - 1) / best;
 }
 
 // Full-array elementwise helpers (Fortran whole-array statements).
@@ -528,35 +534,39 @@ void calc_s_stages(Run<R>& run, int dt_slot) {
   const bool limiter = run.p.heat_flux_limiter != 0;
   const bool pip = run.pip;
   auto xia = run.a.xi;  // per-cell xi_n when partially ionised
-  LARE_BOXW(run, 2, -1, nx + 2, -1, ny + 2, -1, nz + 2, [=] __device__(int ix, int iy, int iz) {
-    const R x = pip ? xia(ix, iy, iz) : xi;
-    temperature(ix, iy, iz) = (g - R(1)) / (R(2) - x) * (energy(ix, iy, iz) - (R(1) - x) * ip);
-  });
-  LARE_BOXW(run, 3, 0, nx, 0, ny, 0, nz, [=] __device__(int ix, int iy, int iz) {
-    if (!limiter) { larsen(ix, iy, iz) = R(1); return; }
-    int ixm = ix - 1, ixp = ix + 1, iym = iy - 1, iyp = iy + 1, izm = iz - 1, izp = iz + 1;
-    R T = temperature(ix, iy, iz);
-    R temp = pow25(T);
-    R q_fs = fl * R(42.85) * rho(ix, iy, iz) * pow15(T);
-    R q_fs2 = q_fs * q_fs;
-    R q_spx = -k0 * temp * (temperature(ixp, iy, iz) - temperature(ixm, iy, iz)) * R(0.5) / dxb(ix);
-    R q_spy = -k0 * temp * (temperature(ix, iyp, iz) - temperature(ix, iym, iz)) * R(0.5) / dyb(iy);
-    R q_spz = -k0 * temp * (temperature(ix, iy, izp) - temperature(ix, iy, izm)) * R(0.5) / dzb(iz);
-    R q_sp2 = q_spx * q_spx + q_spy * q_spy + q_spz * q_spz;
-    larsen(ix, iy, iz) = q_fs / sqrt(q_fs2 + q_sp2);
-  });
   unsigned long long* us = run.us;
-  box_min<1>(run, "parabolic_dt_min", 1, nx, 1, ny, 1, nz, [=] __device__(int ix, int iy, int iz, double* v) {
-    R kappa1 = k0 * larsen(ix, iy, iz);
-    const R x = pip ? xia(ix, iy, iz) : xi;
-    R temp = (g - R(1)) / (R(2) - x) * (energy(ix, iy, iz) - (R(1) - x) * ip);
-    R tp = pow25(temp);
-    R r = rho(ix, iy, iz);
-    R dt1 = r * (dxb(ix) * dxb(ix)) / (R(2) * kappa1 * tp);
-    R dt2 = r * (dyb(iy) * dyb(iy)) / (R(2) * kappa1 * tp);
-    R dt3 = r * (dzb(iz) * dzb(iz)) / (R(2) * kappa1 * tp);
-    v[0] = (double)fmin(fmin(dt1, dt2), dt3);
-  }, U_DTPARAB);
+  const R tc = (g - R(1)) / (R(2) - xi), te0 = (R(1) - xi) * ip;
+  const A1<R> rdx = run.a.rdb[0], rdy = run.a.rdb[1], rdz = run.a.rdb[2];
+  // one pass: the temperature over the whole cell box, the Larsen factor over
+  // 0:n and the explicit limit over 1:n (three passes took 0.236 against
+  // 0.199 ms at 256^3 in FP32)
+  box_min<1>(run, "parabolic_dt_min", -1, nx + 2, -1, ny + 2, -1, nz + 2, [=] __device__(int ix, int iy, int iz, double* v) {
+    auto temp_at = [&](int i, int j, int k) {
+      if (!pip) return tc * (energy(i, j, k) - te0);
+      const R x = xia(i, j, k);
+      return (g - R(1)) / (R(2) - x) * (energy(i, j, k) - (R(1) - x) * ip);
+    };
+    const R T = temp_at(ix, iy, iz);
+    temperature(ix, iy, iz) = T;
+    if (ix < 0 || ix > nx || iy < 0 || iy > ny || iz < 0 || iz > nz) return;
+    const R tp = pow25(T), r = rho(ix, iy, iz);
+    R lf = R(1);
+    if (limiter) {
+      R q_fs = fl * R(42.85) * r * pow15(T);
+      R q_fs2 = q_fs * q_fs;
+      const R kt = -k0 * tp * R(0.5);
+      R q_spx = kt * (temp_at(ix + 1, iy, iz) - temp_at(ix - 1, iy, iz)) * rdx(ix);
+      R q_spy = kt * (temp_at(ix, iy + 1, iz) - temp_at(ix, iy - 1, iz)) * rdy(iy);
+      R q_spz = kt * (temp_at(ix, iy, iz + 1) - temp_at(ix, iy, iz - 1)) * rdz(iz);
+      R q_sp2 = q_spx * q_spx + q_spy * q_spy + q_spz * q_spz;
+      lf = qdiv(q_fs, sqrt(q_fs2 + q_sp2));
+    }
+    larsen(ix, iy, iz) = lf;
+    if (ix < 1 || iy < 1 || iz < 1) return;
+    // the least of rho d^2 / (2 kappa T^5/2) over the axes is that of the least d
+    const R d = fmin(fmin(dxb(ix), dyb(iy)), dzb(iz));
+    v[0] = (double)qdiv(r * (d * d), R(2) * (k0 * lf) * tp);
+  }, U_DTPARAB, 4);
   double* sc = run.sc;
   const double mult = run.p.dt_multiplier;
   const bool f32 = sizeof(R) == 4;
@@ -698,6 +708,9 @@ void heat_conduct_sts2(Run<R>& run, int dt_slot) {
       temperature_from(run, Y2);
       temperature_bcs(run);
     }
+    // The last stage writes the energy in place (conduct.f90:409): Y0 is read
+    // at a cell only by the thread that writes it.
+    if (j == s) Y3 = energy;
     rkl2_stage<R, false>(run, __LINE__, temp(Y2), Y2, Y1, energy, Y3, dt_slot, mtj, mj, nj, omn_r, gt);
     if (j < s) {
       GhostBatch<R> bb;
@@ -715,10 +728,10 @@ void heat_conduct_sts2(Run<R>& run, int dt_slot) {
     }
   }
   // The reference leaves temperature = T(Y2 of the last stage) after
-  // temperature_bcs; keep that, then energy(1:n) = Y3(1:n) and energy_bcs.
+  // temperature_bcs; keep that, then energy_bcs.
   {
     auto temperature = A.temperature;
-    A3<R> y2 = Y2, y3 = Y3;
+    A3<R> y2 = Y2;
     if (!pip) {  // (a partially ionised run formed it for the last stage)
       LARE_BOXW(run, 2, -1, nx + 2, -1, ny + 2, -1, nz + 2, [=] __device__(int ix, int iy, int iz) {
         temperature(ix, iy, iz) = tc * (y2(ix, iy, iz) - te0);
@@ -727,7 +740,6 @@ void heat_conduct_sts2(Run<R>& run, int dt_slot) {
       bb.add(run.g_cell_user, temperature.p);
       ghost_flush(run, bb);
     }
-    LARE_BOXW(run, 2, 1, nx, 1, ny, 1, nz, [=] __device__(int ix, int iy, int iz) { energy(ix, iy, iz) = y3(ix, iy, iz); });
   }
   energy_bcs(run);
 }

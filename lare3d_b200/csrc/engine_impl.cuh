@@ -201,7 +201,7 @@ class EngineT : public EngineBase {
     if (cudaFuncSetAttribute(k_lp4_tile<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lp4_smem_bytes<R>()) !=
             cudaSuccess ||
         bs_attributes<R>() != cudaSuccess || me_attributes<R>() != cudaSuccess ||
-        vm_attributes<R>() != cudaSuccess) {
+        vm_attributes<R>() != cudaSuccess || stage_attributes<R>() != cudaSuccess) {
       err = "shared memory attribute";
       return LARE_ECUDA;
     }
