@@ -49,6 +49,12 @@ __device__ __forceinline__ R& elem_ref(R* first, unsigned off) {
   return *reinterpret_cast<R*>(reinterpret_cast<char*>(first) + off);
 }
 
+// The FP64 product build regroups the limiters' expressions (van_leer in
+// engine.cuh, and their like); FP32 keeps the reference's grouping, where a
+// regrouped rounding is 1e-7 of the value.
+template <class R>
+constexpr bool kRegroup = LARE_FAST && sizeof(R) == 8;
+
 template <class R>
 struct Num;
 template <>

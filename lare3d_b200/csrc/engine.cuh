@@ -541,9 +541,11 @@ void calc_s_stages(Run<R>& run, int dt_slot) {
   // 0:n and the explicit limit over 1:n (three passes took 0.236 against
   // 0.199 ms at 256^3 in FP32)
   box_min<1>(run, "parabolic_dt_min", -1, nx + 2, -1, ny + 2, -1, nz + 2, [=] __device__(int ix, int iy, int iz, double* v) {
+    // FP32 keeps the reference's grouping (kRegroup): a rounding here is the
+    // same one at every cell of a uniform grid
     auto temp_at = [&](int i, int j, int k) {
-      if (!pip) return tc * (energy(i, j, k) - te0);
-      const R x = xia(i, j, k);
+      if (kRegroup<R> && !pip) return tc * (energy(i, j, k) - te0);
+      const R x = pip ? xia(i, j, k) : xi;
       return (g - R(1)) / (R(2) - x) * (energy(i, j, k) - (R(1) - x) * ip);
     };
     const R T = temp_at(ix, iy, iz);
@@ -554,18 +556,28 @@ void calc_s_stages(Run<R>& run, int dt_slot) {
     if (limiter) {
       R q_fs = fl * R(42.85) * r * pow15(T);
       R q_fs2 = q_fs * q_fs;
-      const R kt = -k0 * tp * R(0.5);
-      R q_spx = kt * (temp_at(ix + 1, iy, iz) - temp_at(ix - 1, iy, iz)) * rdx(ix);
-      R q_spy = kt * (temp_at(ix, iy + 1, iz) - temp_at(ix, iy - 1, iz)) * rdy(iy);
-      R q_spz = kt * (temp_at(ix, iy, iz + 1) - temp_at(ix, iy, iz - 1)) * rdz(iz);
-      R q_sp2 = q_spx * q_spx + q_spy * q_spy + q_spz * q_spz;
-      lf = qdiv(q_fs, sqrt(q_fs2 + q_sp2));
+      const R dTx = temp_at(ix + 1, iy, iz) - temp_at(ix - 1, iy, iz);
+      const R dTy = temp_at(ix, iy + 1, iz) - temp_at(ix, iy - 1, iz);
+      const R dTz = temp_at(ix, iy, iz + 1) - temp_at(ix, iy, iz - 1);
+      if (kRegroup<R>) {
+        const R kt = -k0 * tp * R(0.5);
+        const R q_spx = kt * dTx * rdx(ix), q_spy = kt * dTy * rdy(iy), q_spz = kt * dTz * rdz(iz);
+        lf = qdiv(q_fs, sqrt(q_fs2 + (q_spx * q_spx + q_spy * q_spy + q_spz * q_spz)));
+      } else {
+        R q_spx = -k0 * tp * dTx * R(0.5) / dxb(ix);
+        R q_spy = -k0 * tp * dTy * R(0.5) / dyb(iy);
+        R q_spz = -k0 * tp * dTz * R(0.5) / dzb(iz);
+        R q_sp2 = q_spx * q_spx + q_spy * q_spy + q_spz * q_spz;
+        lf = q_fs / sqrt(q_fs2 + q_sp2);
+      }
     }
     larsen(ix, iy, iz) = lf;
     if (ix < 1 || iy < 1 || iz < 1) return;
+    const R kappa1 = k0 * lf;
     // the least of rho d^2 / (2 kappa T^5/2) over the axes is that of the least d
     const R d = fmin(fmin(dxb(ix), dyb(iy)), dzb(iz));
-    v[0] = (double)qdiv(r * (d * d), R(2) * (k0 * lf) * tp);
+    const R top = r * (d * d), bottom = R(2) * kappa1 * tp;
+    v[0] = (double)(kRegroup<R> ? qdiv(top, bottom) : top / bottom);
   }, U_DTPARAB, 4);
   double* sc = run.sc;
   const double mult = run.p.dt_multiplier;
@@ -791,7 +803,6 @@ __device__ __forceinline__ LimOut<R> limiter_dv(R v_advect, R fm, R fi, R fp, R 
   L.Di = L.sign_v * ss * fmin(fmin(fabs(Da) * L.dxbu, fabs(dfi)), fabs(dfu));
   return L;
 }
-#if LARE_FAST
 // The product build's limited flux per unit mass or area moved, in terms of
 // the faces' differences d and slopes s = |d| / dxc (faces below, at and
 // above c): the reference's expressions regrouped, with the upwind choices
@@ -828,7 +839,6 @@ __device__ __forceinline__ R van_leer(R v, R vdt, R f0, R fp, R dm, R d0, R dp, 
   const R D = signed_min(m, d0, du, v);
   return ((up ? f0 : fp) + D * (R(1) - phi)) * vdt;
 }
-#endif
 // The same with plain divisors.
 template <class R>
 __device__ __forceinline__ LimOut<R> limiter(R v_advect, R fm, R fi, R fp, R fp2, R dxci, R dxcm, R dxcp, R dxbi,

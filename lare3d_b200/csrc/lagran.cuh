@@ -790,9 +790,15 @@ void predictor_corrector_step(Run<R>& run) {
     auto vxf = [&](int q) { return (vx[q] + vx[q - sx] + vx[q - sxy] + vx[q - sx - sxy]) * R(0.25); };
     auto vyf = [&](int q) { return (vy[q] + vy[q - 1] + vy[q - sxy] + vy[q - 1 - sxy]) * R(0.25); };
     auto vzf = [&](int q) { return (vz[q] + vz[q - 1] + vz[q - sx] + vz[q - 1 - sx]) * R(0.25); };
+#if LARE_FAST
+    const R tx = (vxf(c) - vxf(c - 1)) * rmx(ix);
+    const R ty = (vyf(c) - vyf(c - sx)) * rmy(iy);
+    const R tz = (vzf(c) - vzf(c - sxy)) * rmz(iz);
+#else
     const R tx = div_rcp(vxf(c) - vxf(c - 1), mx(ix), rmx(ix));
     const R ty = div_rcp(vyf(c) - vyf(c - sx), my(iy), rmy(iy));
     const R tz = div_rcp(vzf(c) - vzf(c - sxy), mz(iz), rmz(iz));
+#endif
     const R tt = last_axis == 0 ? ty + tz + tx : (last_axis == 1 ? tx + tz + ty : tx + ty + tz);
     const R cvc = cv[c];
     const R cv1c = cvc * (R(1) + tt * dt2);

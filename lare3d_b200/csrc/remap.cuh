@@ -218,30 +218,40 @@ __device__ __forceinline__ void mom_flux_vals(R area, R va0, R va1, R rvc, R rvp
   const R phi = fabs(v_advect) * dt / dxbu;
   const R dmu = fabs(dmc) / area / dxbu / rhou;
 #endif
-#if LARE_FAST
-  // the slopes' factors, the widths and the 1/6 in, also shared
+  // kRegroup: the slopes' factors, the widths and the 1/6 in, also shared
   const bool up = !signbit(v_advect);
-  const R dxb6 = dxbu * (R(1) / R(6));
-  const R k0 = (R(2) - phi) * rci * dxb6, ku = (R(1) + phi) * rcu * dxb6, omd = R(1) - dmu;
+  R k0 = R(0), ku = R(0), omd = R(0);
+#if LARE_FAST
+  if constexpr (kRegroup<R>) {
+    const R dxb6 = dxbu * (R(1) / R(6));
+    k0 = (R(2) - phi) * rci * dxb6;
+    ku = (R(1) + phi) * rcu * dxb6;
+    omd = R(1) - dmu;
+  }
 #endif
 #pragma unroll
   for (int comp = 0; comp < 3; ++comp) {
     const R fm = w[comp][0], fi = w[comp][1], fp = w[comp][2], fp2 = w[comp][3];
     const R dfm = fi - fm, dfi = fp - fi, dfp = fp2 - fp;
+    R f;
+    if constexpr (kRegroup<R>) {
+      const R dfu = up ? dfm : dfp;
+      const R da = k0 * fabs(dfi) + ku * fabs(dfu);
+      const R Di = signed_min(lesser(lesser(R(fabs(da)), R(fabs(dfi))), R(fabs(dfu))), dfi, dfu, v_advect);
+      f = (up ? fi : fp) + Di * omd;
+    } else {
+      const R fu = fi * vad_p + fp * vad_m;
+      const R dfu = dfm * vad_p + dfp * vad_m;
 #if LARE_FAST
-    const R dfu = up ? dfm : dfp;
-    const R da = k0 * fabs(dfi) + ku * fabs(dfu);
-    const R Di = signed_min(lesser(lesser(R(fabs(da)), R(fabs(dfi))), R(fabs(dfu))), dfi, dfu, v_advect);
-    const R f = (up ? fi : fp) + Di * omd;
+      R Da = (R(2) - phi) * fabs(dfi) * rci + (R(1) + phi) * fabs(dfu) * rcu;
 #else
-    const R fu = fi * vad_p + fp * vad_m;
-    const R dfu = dfm * vad_p + dfp * vad_m;
-    R Da = (R(2) - phi) * fabs(dfi) / dxci + (R(1) + phi) * fabs(dfu) / dxcu;
-    Da = Da * (R(1) / R(6));
-    const R ss = R(0.5) * (copysign(R(1), dfi) + copysign(R(1), dfu));
-    const R Di = sign_v * ss * fmin(fmin(fabs(Da) * dxbu, fabs(dfi)), fabs(dfu));
-    const R f = fu + Di * (R(1) - dmu);
+      R Da = (R(2) - phi) * fabs(dfi) / dxci + (R(1) + phi) * fabs(dfu) / dxcu;
 #endif
+      Da = Da * (R(1) / R(6));
+      const R ss = R(0.5) * (copysign(R(1), dfi) + copysign(R(1), dfu));
+      const R Di = sign_v * ss * fmin(fmin(fabs(Da) * dxbu, fabs(dfi)), fabs(dfu));
+      f = fu + Di * (R(1) - dmu);
+    }
     if constexpr (BOTH) fpre[comp] = f;
     F[comp] = f * dmc;
   }

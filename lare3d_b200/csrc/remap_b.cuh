@@ -54,64 +54,60 @@ struct BSArgs {
 
 // One transported component's four-point window along the sweep axis:
 // B / dbv and dbv (in the carried divisor form) at c, c + e_A, c + 2 e_A, and
-// what the limiter takes of the faces below, at and above c.  The exact
-// builds keep B / dbv at c - e_A and evaluate the reference's expressions; the
-// product build carries each face's difference and its slope |d| / dc1,
-// formed once when the face enters the window instead of once for each of
-// the three fluxes that read it.
+// what the limiter takes of the faces below, at and above c: B / dbv at
+// c - e_A and dc1, for the reference's expressions, or (kRegroup) each face's
+// difference and its slope |d| / dc1, formed once when the face enters the
+// window instead of once for each of the three fluxes that read it.
 template <class R>
 struct BWin {
   R q0, qp, qp2, v0, vp, vp2;
-#if LARE_FAST
-  R dm, d0, dp, sm, s0, sp;
-#else
-  R qm, dcm, dc0, dcp;
-#endif
+  R dm, d0, dp, sm, s0, sp;  // kRegroup
+  R qm, dcm, dc0, dcp;       // else
   // the points c - e_A (or c where the stencil is clamped) and c, and dc1 below c
   __device__ __forceinline__ void start(R qm_, R q0_, R v0_, R dcm_) {
     q0 = q0_;
     v0 = v0_;
-#if LARE_FAST
-    dm = q0_ - qm_;
-    sm = fabs(dm) * fast_rcp(dcm_);
-#else
-    qm = qm_;
-    dcm = dcm_;
-#endif
+    if constexpr (kRegroup<R>) {
+      dm = q0_ - qm_;
+      sm = fabs(dm) * fast_rcp(dcm_);
+    } else {
+      qm = qm_;
+      dcm = dv_of(dcm_);
+    }
   }
   // the point c + e_A, and dc1 at c
   __device__ __forceinline__ void next(R q, R v, R dc) {
     qp = q;
     vp = v;
-#if LARE_FAST
-    d0 = q - q0;
-    s0 = fabs(d0) * fast_rcp(dc);
-#else
-    dc0 = dc;
-#endif
+    if constexpr (kRegroup<R>) {
+      d0 = q - q0;
+      s0 = fabs(d0) * fast_rcp(dc);
+    } else {
+      dc0 = dv_of(dc);
+    }
   }
   // the point c + 2 e_A, and dc1 at c + e_A (in the carried divisor form)
   __device__ __forceinline__ void top(R q, R v, R dc) {
     qp2 = q;
     vp2 = v;
-#if LARE_FAST
-    dp = q - qp;
-    sp = fabs(dp) * dc;
-#else
-    dcp = dc;
-#endif
+    if constexpr (kRegroup<R>) {
+      dp = q - qp;
+      sp = fabs(dp) * dc;
+    } else {
+      dcp = dc;
+    }
   }
   __device__ __forceinline__ void shift() {
-#if LARE_FAST
-    dm = d0;
-    d0 = dp;
-    sm = s0;
-    s0 = sp;
-#else
-    qm = q0;
-    dcm = dc0;
-    dc0 = dcp;
-#endif
+    if constexpr (kRegroup<R>) {
+      dm = d0;
+      d0 = dp;
+      sm = s0;
+      s0 = sp;
+    } else {
+      qm = q0;
+      dcm = dc0;
+      dc0 = dcp;
+    }
     q0 = qp;
     qp = qp2;
     v0 = vp;
@@ -119,12 +115,12 @@ struct BWin {
   }
   // the flux at c: db1 at c and c + e_A
   __device__ __forceinline__ R flux(R v_advect, R db0, R dbp, R dt) const {
-#if LARE_FAST
-    return van_leer(v_advect, v_advect * dt, q0, qp, dm, d0, dp, sm, s0, sp, db0, dbp, v0, vp);
-#else
-    const LimOut<R> L = limiter_dv<R>(v_advect, qm, q0, qp, qp2, dc0, dcm, dcp, db0, dbp, v0, vp, dt, true);
-    return (L.fu + L.Di * (R(1) - L.phi)) * v_advect * dt;
-#endif
+    if constexpr (kRegroup<R>) {
+      return van_leer(v_advect, v_advect * dt, q0, qp, dm, d0, dp, sm, s0, sp, db0, dbp, v0, vp);
+    } else {
+      const LimOut<R> L = limiter_dv<R>(v_advect, qm, q0, qp, qp2, dc0, dcm, dcp, db0, dbp, v0, vp, dt, true);
+      return (L.fu + L.Di * (R(1) - L.phi)) * v_advect * dt;
+    }
   }
 };
 
@@ -515,14 +511,14 @@ __global__ void __launch_bounds__(32 * kBsY, sizeof(R) == 8 ? 2 : 4) k_bsweep_x(
       const R qp = __shfl_down_sync(all, q, 1), dd = __shfl_down_sync(all, d, 1);
       qm = left ? qm : q;
       qp2 = right ? qp2 : qp;
-#if LARE_FAST
-      const R em = q - qm, e0_ = qp - q, ep = qp2 - qp;
-      return van_leer(v, v * dt, q, qp, em, e0_, ep, R(fabs(em) * dcm), R(fabs(e0_) * dc), R(fabs(ep) * dcp), db, dbp,
-                      d, dd);
-#else
-      const LimOut<R> M = limiter_dv<R>(v, qm, q, qp, qp2, dc, dcm, dcp, db, dbp, d, dd, dt, true);
-      return (M.fu + M.Di * (R(1) - M.phi)) * v * dt;
-#endif
+      if constexpr (kRegroup<R>) {
+        const R em = q - qm, e0_ = qp - q, ep = qp2 - qp;
+        return van_leer(v, v * dt, q, qp, em, e0_, ep, R(fabs(em) * dcm), R(fabs(e0_) * dc), R(fabs(ep) * dcp), db,
+                        dbp, d, dd);
+      } else {
+        const LimOut<R> M = limiter_dv<R>(v, qm, q, qp, qp2, dc, dcm, dcp, db, dbp, d, dd, dt, true);
+        return (M.fu + M.Di * (R(1) - M.phi)) * v * dt;
+      }
     };
     const R f1 = flux((v0.c + vm.c) * R(0.5), q1, d1);
     f1s[iz & 1][ty][lane] = f1;

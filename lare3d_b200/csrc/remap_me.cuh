@@ -94,7 +94,11 @@ __device__ __forceinline__ void me_volumes(const MEArgs<R>& g, const R (&dv)[3],
                                            R& c1, R& c2) {
   constexpr int T1 = A == 0 ? 1 : 0, T2 = A == 2 ? 1 : 2;
   const int pp[3] = {ix, iy, iz};
+#if LARE_FAST
+  auto quot = [&](R a, int d) { return a * g.r[d](pp[d]); };
+#else
   auto quot = [&](R a, int d) { return div_rcp(a, g.m[d](pp[d]), g.r[d](pp[d])); };
+#endif
   const R t1 = H1 ? quot(dv[T1], T1) : R(0), t2 = H2 ? quot(dv[T2], T2) : R(0);
   const R t12 = t1 + t2;
   c1 = cv * (R(1) + (t12 + quot(dv[A], A)) * dt);
@@ -142,30 +146,26 @@ struct Tr2 {
 template <class R>
 struct MEFace {
   R vf, dt, area;
-#if LARE_FAST
   bool up;
-  R phi, dxb, dxb6, vd0, vdu;
-#else
-  R vdc[3], db0, dbp;
-#endif
+  R phi, dxb, dxb6, vd0, vdu;  // kRegroup
+  R vdc[3], db0, dbp;          // else
   __device__ __forceinline__ MEFace(const R (&vdc_)[3], R db0_, R dbp_, R vf_, R dt_, R area_)
       : vf(vf_), dt(dt_), area(area_) {
-#if LARE_FAST
-    up = !signbit(vf);
-    dxb = up ? db0_ : dbp_;
-    phi = fabs(vf) * dt * fast_rcp(dxb);
-    dxb6 = dxb * (R(1) / R(6));
-    vd0 = vdc_[1];
-    vdu = up ? vdc_[0] : vdc_[2];
-#else
-    db0 = db0_;
-    dbp = dbp_;
-    vdc[0] = vdc_[0];
-    vdc[1] = vdc_[1];
-    vdc[2] = vdc_[2];
-#endif
+    if constexpr (kRegroup<R>) {
+      up = !signbit(vf);
+      dxb = up ? db0_ : dbp_;
+      phi = fabs(vf) * dt * fast_rcp(dxb);
+      dxb6 = dxb * (R(1) / R(6));
+      vd0 = vdc_[1];
+      vdu = up ? vdc_[0] : vdc_[2];
+    } else {
+      db0 = db0_;
+      dbp = dbp_;
+      vdc[0] = vdc_[0];
+      vdc[1] = vdc_[1];
+      vdc[2] = vdc_[2];
+    }
   }
-#if LARE_FAST
   // upwind value and limited difference
   __device__ __forceinline__ R limited(const R (&f)[4], R& fu) const {
     const R dm = f[1] - f[0], d0 = f[2] - f[1], dp = f[3] - f[2];
@@ -174,29 +174,35 @@ struct MEFace {
     const R da = (R(2) - phi) * (fabs(d0) * vd0) + (R(1) + phi) * (fabs(du) * vdu);
     return signed_min(lesser(lesser(R(fabs(da) * dxb6), R(fabs(d0))), R(fabs(du))), d0, du, vf);
   }
-#endif
+  __device__ __forceinline__ LimOut<R> plain(const R (&f)[4]) const {
+    return limiter_dv<R>(vf, f[0], f[1], f[2], f[3], vdc[1], vdc[0], vdc[2], db0, dbp, R(0), R(0), dt, false);
+  }
   __device__ __forceinline__ R mass(const R (&r)[4]) const {
-#if LARE_FAST
-    R fu;
-    const R D = limited(r, fu);
-    return (fu + D * (R(1) - phi)) * vf * dt * area;
-#else
-    const LimOut<R> L = limiter_dv<R>(vf, r[0], r[1], r[2], r[3], vdc[1], vdc[0], vdc[2], db0, dbp, R(0), R(0), dt, false);
-    return (L.fu + L.Di * (R(1) - L.phi)) * vf * dt * area;
-#endif
+    if constexpr (kRegroup<R>) {
+      R fu;
+      const R D = limited(r, fu);
+      return (fu + D * (R(1) - phi)) * vf * dt * area;
+    } else {
+      const LimOut<R> L = plain(r);
+      return (L.fu + L.Di * (R(1) - L.phi)) * vf * dt * area;
+    }
   }
   __device__ __forceinline__ R energy(const R (&e)[4], R r0, R rp, R dm) const {
+    if constexpr (kRegroup<R>) {
+      R fu;
+      const R D = limited(e, fu);
+      const R dmu = fabs(dm) * fast_rcp(area * dxb * (up ? r0 : rp));
+      return (fu + D * (R(1) - dmu)) * dm;
+    } else {
+      const LimOut<R> L = plain(e);
+      const R rhou = r0 * L.vad_p + rp * L.vad_m;
 #if LARE_FAST
-    R fu;
-    const R D = limited(e, fu);
-    const R dmu = fabs(dm) * fast_rcp(area * dxb * (up ? r0 : rp));
-    return (fu + D * (R(1) - dmu)) * dm;
+      const R dmu = fabs(dm) * fast_rcp(area * L.dxbu * rhou);
 #else
-    const LimOut<R> L = limiter_dv<R>(vf, e[0], e[1], e[2], e[3], vdc[1], vdc[0], vdc[2], db0, dbp, R(0), R(0), dt, false);
-    const R rhou = r0 * L.vad_p + rp * L.vad_m;
-    const R dmu = fabs(dm) / area / L.dxbu / rhou;
-    return (L.fu + L.Di * (R(1) - dmu)) * dm;
+      const R dmu = fabs(dm) / area / L.dxbu / rhou;
 #endif
+      return (L.fu + L.Di * (R(1) - dmu)) * dm;
+    }
   }
 };
 
