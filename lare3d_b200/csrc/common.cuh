@@ -354,7 +354,14 @@ __global__ void __launch_bounds__(256) k_box_min(int i0, int j0, int k0, int ni,
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   int j = blockIdx.y * blockDim.y + threadIdx.y;
   double v[NV];
-  for (int q = 0; q < NV; ++q) v[q] = DBL_MAX;
+  // from the minima recorded so far (any recorded value bounds the final one),
+  // which fn may use to leave out a point that cannot lower them; read by one
+  // warp, since every warp's read of the one line took longer than the points
+  __shared__ double rec[NV];
+  if (threadIdx.y == 0 && threadIdx.x < NV)
+    rec[threadIdx.x] = __longlong_as_double(*(volatile long long*)(out + threadIdx.x));
+  __syncthreads();
+  for (int q = 0; q < NV; ++q) v[q] = rec[q];
   // `planes` consecutive planes per block (the min does not depend on the
   // order), so that few blocks contend for the atomic on the result
   if (i < ni && j < nj) {
@@ -362,7 +369,7 @@ __global__ void __launch_bounds__(256) k_box_min(int i0, int j0, int k0, int ni,
     for (int kk = kb; kk < kb + planes && kk < nk; ++kk) {
       double w[NV];
       for (int q = 0; q < NV; ++q) w[q] = DBL_MAX;
-      fn(i0 + i, j0 + j, k0 + kk, w);
+      fn(i0 + i, j0 + j, k0 + kk, w, v);
       for (int q = 0; q < NV; ++q) v[q] = fmin(v[q], w[q]);
     }
   }

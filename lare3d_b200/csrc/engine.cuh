@@ -329,10 +329,11 @@ template <int NV, class R, class Fn>
 inline void box_min(Run<R>& run, const char* site, int i0, int i1, int j0, int j1, int k0, int k1, Fn fn, int uslot,
                     int words = 0) {
   int ni = i1 - i0 + 1, nj = j1 - j0 + 1, nk = k1 - k0 + 1;
-  // planes per block: fewer blocks contend for the atomic, at the cost of
-  // resident warps; measured at 256^3: 8 in FP32 (0.23 -> 0.18 ms for set_dt),
-  // 1 in FP64 (8 took 0.38 -> 0.42 ms)
-  constexpr int kMinPlanes = sizeof(R) == 4 ? 8 : 1;
+  // planes per block: fewer blocks contend for the atomic, and later blocks
+  // find lower minima recorded (set_dt leaves out most cells by them).  At
+  // 256^3 in FP64 1 plane takes 0.52 ms for set_dt, 4 0.41, 8 0.35 and 12
+  // 0.35; at 80^3 8 take 29 us and 12 34.  FP32: 0.23 -> 0.18 ms from 1 to 8.
+  constexpr int kMinPlanes = 8;
   dim3 blk(64, 4, 1);
   dim3 grd((ni + 63) / 64, (nj + 3) / 4, (nk + kMinPlanes - 1) / kMinPlanes);
   int k = run.prof_begin(site, 0, words, (double)ni * nj * nk);
@@ -540,7 +541,7 @@ void calc_s_stages(Run<R>& run, int dt_slot) {
   // one pass: the temperature over the whole cell box, the Larsen factor over
   // 0:n and the explicit limit over 1:n (three passes took 0.236 against
   // 0.199 ms at 256^3 in FP32)
-  box_min<1>(run, "parabolic_dt_min", -1, nx + 2, -1, ny + 2, -1, nz + 2, [=] __device__(int ix, int iy, int iz, double* v) {
+  box_min<1>(run, "parabolic_dt_min", -1, nx + 2, -1, ny + 2, -1, nz + 2, [=] __device__(int ix, int iy, int iz, double* v, const double*) {
     // FP32 keeps the reference's grouping (kRegroup): a rounding here is the
     // same one at every cell of a uniform grid
     auto temp_at = [&](int i, int j, int k) {
