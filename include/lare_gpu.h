@@ -389,6 +389,16 @@ int lare_gpu_check_division(const double* a, const double* b, long long n, doubl
  */
 int lare_gpu_check_reciprocal(const double* b, long long n, double* out, void* stream);
 
+/*
+ * Self-check of the kernels that copy by tensor maps: runs each of their
+ * launchers, in the given precision, on a context that cannot make a map, and
+ * stores the number of kernels launched, which must be 0 (a kernel given an
+ * unset map copies from wherever its bytes say).  Returns LARE_ECUDA, the
+ * status that such a context's calls return.  Host only; needs no GPU.  No
+ * counterpart in the reference.
+ */
+int lare_gpu_check_unmapped(int precision, long long* launches);
+
 void lare_gpu_destroy(lare_ctx* ctx);
 
 /*

@@ -23,8 +23,6 @@
 //   +Fz(c-ez), +Fy(c-ey), +Fx(c-ex), -Fx(c), -Fy(c), -Fz(c).
 #pragma once
 
-#include "tma.cuh"
-
 LARE_BEGIN
 
 constexpr int kCTY = 8, kCZ = 32;             // rows of a CTA tile, largest chunk of z (march_chunk)
@@ -342,7 +340,7 @@ void rkl2_stage(Run<R>& run, int line, const TempOf<R>& T, A3<R> y2, A3<R> y1, A
   StageMaps maps;
   const long long f = 2 + 2LL * run.sx + 2LL * run.sxy;
   const auto map = [&](CUtensorMap* m, const A3<R>& x, int rows) {
-    if (!tma_map(m, (const R*)x.p - f, run.n, run.sx, run.sxy, L::W, rows, 1)) run.launch_error = true;
+    make_map(run, m, (const R*)x.p - f, L::W, rows, 1);
   };
   map(&maps.T, T.y, kCTY + 2);
   for (int q = 0; q < 9; ++q) map(&maps.k[q], run.a.kf[q], q / 3 == 1 ? kCTY + 1 : kCTY);
@@ -350,6 +348,7 @@ void rkl2_stage(Run<R>& run, int line, const TempOf<R>& T, A3<R> y2, A3<R> y1, A
   map(&maps.y0, y0, kCTY);
   map(&maps.y1, y1, kCTY);
   map(&maps.lc0, run.a.Lc_Y0, kCTY);
+  if (run.launch_error) return;
   dim3 grid((nx + kSTX - 1) / kSTX, (ny + kCTY - 1) / kCTY, 1);
   a.chunk = march_chunk(nz, grid.x * grid.y, kCZ, resident_blocks<k_rkl2_stage<R, FIRST>>(32 * kCTY, L::smem));
   grid.z = (nz + a.chunk - 1) / a.chunk;

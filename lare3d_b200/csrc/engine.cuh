@@ -26,6 +26,7 @@
 
 #include "../../include/lare_gpu.h"
 #include "common.cuh"
+#include "tma.cuh"
 
 LARE_BEGIN
 
@@ -125,7 +126,8 @@ struct Run {
   int peak_substeps = 0, last_substeps = 0, steps_taken = 0, n_s_stages = 0;
   int blk_x = 32, blk_y = 4;            // block shape of the point kernels (measured best at 256^3)
   bool capturing = false;               // recording a CUDA graph of whole steps
-  bool launch_error = false;            // a tensor map could not be made
+  PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;  // tma_encoder(), set by init
+  bool launch_error = false;            // a tensor map could not be made: no kernel that copies by one is launched
   cudaStream_t s_body = nullptr;        // captures the body of the resistive sub-cycle loop
   GSpec g_cell, g_node, g_bx, g_by, g_bz, g_cell_mpi, g_cell_user, g_dm[3];
   Prof prof;
@@ -340,6 +342,15 @@ inline void box_min(Run<R>& run, const char* site, int i0, int i1, int j0, int j
   k_box_min<NV><<<grd, blk, 0, run.s>>>(i0, j0, k0, ni, nj, nk, kMinPlanes, fn, run.us + uslot);
   run.prof_end(k);
   ++run.launches;
+}
+
+// The map of array a (from its first element) with boxes of bx x by x bz, for a
+// kernel that copies by it.  Where it cannot be made run.launch_error stays
+// set, and the launcher returns without launching: a kernel given an unset map
+// copies from whatever the map's bytes say.
+template <class R>
+inline void make_map(Run<R>& run, CUtensorMap* m, const R* first, int bx, int by, int bz) {
+  if (!tma_map(run.encode, m, first, run.n, run.sx, run.sxy, bx, by, bz)) run.launch_error = true;
 }
 
 // ---------------------------------------------------------------------

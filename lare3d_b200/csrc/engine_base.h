@@ -56,4 +56,9 @@ EngineBase* make_engine_f64_exact(const lare_params* p, int nx, int ny, int nz, 
 EngineBase* make_engine_f32(const lare_params* p, int nx, int ny, int nz, const double* const* metrics6,
                             std::string& err);
 
+// lare_gpu_check_unmapped of one precision.
+int check_unmapped_f64(long long* launches);
+int check_unmapped_f64_exact(long long* launches);
+int check_unmapped_f32(long long* launches);
+
 }  // namespace lare

@@ -10,4 +10,5 @@ EngineBase* make_engine_f32(const lare_params* p, int nx, int ny, int nz, const 
                             std::string& err) {
   return make_engine<float>(p, nx, ny, nz, metrics6, err);
 }
+int check_unmapped_f32(long long* launches) { return check_unmapped<float>(launches); }
 }  // namespace lare

@@ -11,4 +11,5 @@ EngineBase* make_engine_f64_exact(const lare_params* p, int nx, int ny, int nz, 
                                   std::string& err) {
   return make_engine<double>(p, nx, ny, nz, metrics6, err);
 }
+int check_unmapped_f64_exact(long long* launches) { return check_unmapped<double>(launches); }
 }  // namespace lare

@@ -12,4 +12,5 @@ EngineBase* make_engine_f64(const lare_params* p, int nx, int ny, int nz, const 
                             std::string& err) {
   return make_engine<double>(p, nx, ny, nz, metrics6, err);
 }
+int check_unmapped_f64(long long* launches) { return check_unmapped<double>(launches); }
 }  // namespace lare

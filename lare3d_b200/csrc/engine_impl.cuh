@@ -197,6 +197,8 @@ class EngineT : public EngineBase {
     run.elems = (size_t)elems;
     const long long off = 2 + 2LL * run.sx + 2LL * sxy;
     if (cudaStreamCreateWithFlags(&run.s, cudaStreamNonBlocking) != cudaSuccess) { err = "stream"; return LARE_ECUDA; }
+    run.encode = tma_encoder();
+    if (!run.encode) { err = "cuTensorMapEncodeTiled is missing"; return LARE_ECUDA; }
     // kernels with more than the default 48 KiB of dynamic shared memory
     if (cudaFuncSetAttribute(k_lp4_tile<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lp4_smem_bytes<R>()) !=
             cudaSuccess ||
@@ -668,6 +670,60 @@ class EngineT : public EngineBase {
   const char* error() const override { return run.err.c_str(); }
   void set_error(const std::string& e) override { run.err = e; }
 };
+
+// Every launcher of a kernel that copies by tensor maps, on a context that
+// cannot make one: the number of kernels launched has to stay 0.
+template <class R>
+int check_unmapped(long long* launches) {
+  Run<R> run{};
+  run.n[0] = run.n[1] = run.n[2] = 8;
+  run.sx = 16;
+  run.sxy = 16 * 13;
+  std::vector<R> none((size_t)run.sxy * 13);
+  const A3<R> a{none.data() + 2 + 2 * run.sx + 2 * run.sxy, run.sx, run.sxy};
+  R* const b[3] = {a.p, a.p, a.p};
+  const auto fresh = [&] { return std::exchange(run.launch_error, false); };
+  bool flagged = true;
+  const auto sweep = [&](auto axis) {
+    constexpr int A = decltype(axis)::value;
+    for (int mode = 0; mode < 3; ++mode) {
+      bsweep<A>(run, a.p, b, b, SC_DT, mode);
+      flagged &= fresh();
+    }
+    for (int q = 0; q < 4; ++q) {
+      MEArgs<R> me{};
+      for (int d = 0; d < 3; ++d) {
+        me.v[d] = a.p;
+        me.pass[d] = 1;
+      }
+      me.pass[A == 0 ? 1 : 0] = q & 1;
+      me.pass[A == 2 ? 1 : 2] = q >> 1;
+      me.rho = me.energy = me.cv = me.rho_new = me.energy_new = me.dm = me.cv1 = me.cv2 = a.p;
+      me.nx = me.ny = me.nz = 8;
+      me.per = true;
+      mass_energy_sweep<A>(run, me, 0);
+      flagged &= fresh();
+    }
+    VMArgs<R> vm{};
+    vm.rho = vm.cv1 = vm.cv2 = vm.dm = vm.m.va = a.p;
+    for (int d = 0; d < 3; ++d) vm.m.v[d] = vm.m.vn[d] = a.p;
+    vm.m.nx = vm.m.ny = vm.m.nz = vm.m.na = vm.m.n3 = 8;
+    vm_launch<A>(run, vm);
+    flagged &= fresh();
+  };
+  sweep(std::integral_constant<int, 0>());
+  sweep(std::integral_constant<int, 1>());
+  sweep(std::integral_constant<int, 2>());
+  run.a.Lc_Y0 = run.a.rho = a;
+  for (A3<R>& k : run.a.kf) k = a;
+  const TempOf<R> T{a, R(1), R(0)};
+  rkl2_stage<R, true>(run, 0, T, a, a, a, a, SC_DT, R(0), R(0), R(0), R(0), R(0));
+  flagged &= fresh();
+  rkl2_stage<R, false>(run, 0, T, a, a, a, a, SC_DT, R(0), R(0), R(0), R(0), R(0));
+  flagged &= fresh();
+  *launches = run.launches;
+  return flagged ? LARE_ECUDA : LARE_OK;
+}
 
 template <class R>
 EngineBase* make_engine(const lare_params* p, int nx, int ny, int nz, const double* const* metrics6,

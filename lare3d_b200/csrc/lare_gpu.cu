@@ -257,6 +257,14 @@ int lare_gpu_check_reciprocal(const double* b, long long n, double* out, void* s
   return cudaGetLastError() == cudaSuccess ? LARE_OK : LARE_ECUDA;
 }
 
+int lare_gpu_check_unmapped(int precision, long long* launches) {
+  if (!launches) return LARE_EINVAL;
+  if (precision == LARE_FP64) return lare::check_unmapped_f64(launches);
+  if (precision == LARE_FP64_EXACT) return lare::check_unmapped_f64_exact(launches);
+  if (precision == LARE_FP32) return lare::check_unmapped_f32(launches);
+  return LARE_EINVAL;
+}
+
 void* lare_gpu_stream(lare_ctx* c) { return (c && c->e) ? c->e->stream() : nullptr; }
 
 const char* lare_gpu_last_error(lare_ctx* c) {

@@ -553,10 +553,6 @@ void remap_sweep(Run<R>& run, int dt_slot, int pass[3], int bmode) {
     gm.S3 = A == 1 ? sxy : sx;
     const bool rke = run.p.rke != 0;
     for (int q = 0; q < 3; ++q) gm.fp[q] = rke ? Ar.rke_f[q].p : nullptr;
-    // words: fused, v (3), v1, rho, cv1, cv2, dm read and the new v (3) written
-    const char* site = fused_vm ? (A == 0 ? "remap_sweep_vert_mom_x" : "remap_sweep_vert_mom_march")
-                                : (A == 0 ? "remap_sweep_mom_x" : "remap_sweep_mom_march");
-    const int k = run.prof_begin(site, 0, fused_vm ? 11 : (rke ? 17 : 14), (double)(nx + 1) * (ny + 1) * (nz + 1));
     if (fused_vm) {
       VMArgs<R> vm;
       vm.m = gm;
@@ -566,23 +562,27 @@ void remap_sweep(Run<R>& run, int dt_slot, int pass[3], int bmode) {
       vm.cv2 = cv2;
       vm.dm = dm;
       vm_launch<A>(run, vm);
-    } else if (A == 0) {
-      dim3 grd((nx + 1 + 30) / 31, (ny + 1 + 3) / 4, nz + 1);
-      if (rke)
-        k_mom_x<R, true><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
-      else
-        k_mom_x<R, false><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
     } else {
-      dim3 grd((nx + 1 + 31) / 32, (gm.n3 + 1 + 3) / 4, 1);
-      gm.chunk = march_chunk(na + 1, grd.x * grd.y, kMomA, resident_blocks<k_mom_march<R, true>>(128));
-      grd.z = (na + 1 + gm.chunk - 1) / gm.chunk;
-      if (rke)
-        k_mom_march<R, true><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
-      else
-        k_mom_march<R, false><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
+      const int k = run.prof_begin(A == 0 ? "remap_sweep_mom_x" : "remap_sweep_mom_march", 0, rke ? 17 : 14,
+                                   (double)(nx + 1) * (ny + 1) * (nz + 1));
+      if (A == 0) {
+        dim3 grd((nx + 1 + 30) / 31, (ny + 1 + 3) / 4, nz + 1);
+        if (rke)
+          k_mom_x<R, true><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
+        else
+          k_mom_x<R, false><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
+      } else {
+        dim3 grd((nx + 1 + 31) / 32, (gm.n3 + 1 + 3) / 4, 1);
+        gm.chunk = march_chunk(na + 1, grd.x * grd.y, kMomA, resident_blocks<k_mom_march<R, true>>(128));
+        grd.z = (na + 1 + gm.chunk - 1) / gm.chunk;
+        if (rke)
+          k_mom_march<R, true><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
+        else
+          k_mom_march<R, false><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
+      }
+      run.prof_end(k);
+      ++run.launches;
     }
-    run.prof_end(k);
-    ++run.launches;
   }
   if (run.p.rke) {
     // rke (xremap.f90:664-695 and siblings): the old velocities are still

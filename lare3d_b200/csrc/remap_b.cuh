@@ -31,8 +31,6 @@
 // of the arrays' box -2..n+2 is written; the update covers 0..n+1.
 #pragma once
 
-#include "tma.cuh"
-
 LARE_BEGIN
 
 constexpr int kBsY = 8;            // rows of a tile; its first row only hands on its fluxes
@@ -612,21 +610,21 @@ void bsweep(Run<R>& run, R* const va, R* const (&in)[3], R* const (&out)[3], int
   g.nz = run.n[2];
   g.sx = run.sx;
   g.sxy = run.sxy;
+  BSMaps maps;
+  const auto map = [&](CUtensorMap* m, const R* first, int rows) {
+    make_map(run, m, first, BSTile<R>::W, A == 1 ? 1 : rows, A == 1 ? rows : 1);
+  };
+  map(&maps.va, g.va, kBsY + 2);
+  map(&maps.b[0], g.in[0], kBsY);
+  map(&maps.b[1], g.in[A == 0 ? 1 : 3 - A], kBsY);
+  map(&maps.b[2], g.in[A == 0 ? 2 : A], kBsY);
+  if (run.launch_error) return;
   const int nt = (A == 1 ? g.nz : g.ny) + 5;                   // rows: y, or z for the y sweep
   const int nm = (A == 1 ? g.ny : g.nz) + 5;                   // marched axis
   const int xout = A == 0 ? kBsXOut : kBsOut;
   dim3 grd((g.nx + 5 + xout - 1) / xout, (nt + kBsY - 2) / (kBsY - 1), 1);
   g.chunk = march_chunk(nm, grd.x * grd.y, 64, bs_resident<A, R>());
   grd.z = (nm + g.chunk - 1) / g.chunk;
-  BSMaps maps;
-  const auto map = [&](CUtensorMap* m, const R* first, int rows) {
-    if (!tma_map(m, first, run.n, run.sx, run.sxy, BSTile<R>::W, A == 1 ? 1 : rows, A == 1 ? rows : 1))
-      run.launch_error = true;
-  };
-  map(&maps.va, g.va, kBsY + 2);
-  map(&maps.b[0], g.in[0], kBsY);
-  map(&maps.b[1], g.in[A == 0 ? 1 : 3 - A], kBsY);
-  map(&maps.b[2], g.in[A == 0 ? 2 : A], kBsY);
   const double pts = (double)(g.nx + 5) * (g.ny + 5) * (g.nz + 5);
   // words: va and B (3) read, B (3) written.  The sweep that finishes a
   // remap's B (and puts it back from flux form) is a site of its own.

@@ -562,13 +562,13 @@ __global__ void __launch_bounds__(32 * kMeY, sizeof(R) == 8 ? 2 : 4)
 }
 
 template <int A, bool HX, bool HT, class R>
-inline void me_launch(Run<R>& run, MEArgs<R>& g) {
+inline void me_launch(Run<R>& run, MEArgs<R>& g, int words) {
   using L = METile<HX, HT, R>;
   constexpr int T1 = A == 0 ? 1 : 0, T2 = A == 2 ? 1 : 2;
   MEMaps maps;
   const long long f = 2 + 2LL * run.sx + 2LL * run.sxy;
   const auto map = [&](CUtensorMap* m, const R* p, int rows) {
-    if (!tma_map(m, p - f, run.n, run.sx, run.sxy, L::W, A == 1 ? 1 : rows, A == 1 ? rows : 1)) run.launch_error = true;
+    make_map(run, m, p - f, L::W, A == 1 ? 1 : rows, A == 1 ? rows : 1);
   };
   map(&maps.va, g.v[A], kMeY + 1);
   map(&maps.vx, g.v[T1], kMeY + 1);
@@ -576,10 +576,13 @@ inline void me_launch(Run<R>& run, MEArgs<R>& g) {
   map(&maps.rho, g.rho, kMeY);
   map(&maps.energy, g.energy, kMeY);
   map(&maps.cv, g.cv, kMeY);
+  if (run.launch_error) return;
   const int rows = (A == 1 ? g.nz : g.ny) + 4, len = (A == 1 ? g.ny : g.nz) + 4;
   const int xout = A == 0 ? kMeXOut : 32;
   dim3 grd((g.nx + 4 + xout - 1) / xout, (rows + kMeY - 1) / kMeY, 1);
   const dim3 blk(32, kMeY, 1);
+  const int k = run.prof_begin(A == 0 ? "remap_sweep_mass_energy_x" : "remap_sweep_mass_energy_march", 0, words,
+                               (double)(g.nx + 4) * (g.ny + 4) * (g.nz + 4));
   if constexpr (A == 0) {
     if (g.per) {
       k_me_ghost_x<R><<<dim3((4 * (g.ny + 2) + 127) / 128, g.nz + 2), 128, 0, run.s>>>(g);
@@ -593,6 +596,8 @@ inline void me_launch(Run<R>& run, MEArgs<R>& g) {
     grd.z = (len + g.chunk - 1) / g.chunk;
     k_me_march<A, HX, HT, R><<<grd, blk, L::smem, run.s>>>(maps, g);
   }
+  run.prof_end(k);
+  ++run.launches;
 }
 
 // Dynamic shared memory beyond the default 48 KiB, once per context.
@@ -624,19 +629,15 @@ void mass_energy_sweep(Run<R>& run, MEArgs<R> g, int swept) {
   constexpr int T1 = A == 0 ? 1 : 0, T2 = A == 2 ? 1 : 2;
   // words: rho, energy, cv and the velocity components still to come read;
   // dm, rho, energy, cv1 and (but in the third sweep) cv2 written
-  const int k = run.prof_begin(A == 0 ? "remap_sweep_mass_energy_x" : "remap_sweep_mass_energy_march", 0,
-                               swept == 0 ? 11 : (swept == 1 ? 10 : 8),
-                               (double)(g.nx + 4) * (g.ny + 4) * (g.nz + 4));
+  const int words = swept == 0 ? 11 : (swept == 1 ? 10 : 8);
   if (g.pass[T1] && g.pass[T2])
-    me_launch<A, true, true>(run, g);
+    me_launch<A, true, true>(run, g, words);
   else if (g.pass[T1])
-    me_launch<A, true, false>(run, g);
+    me_launch<A, true, false>(run, g, words);
   else if (g.pass[T2])
-    me_launch<A, false, true>(run, g);
+    me_launch<A, false, true>(run, g, words);
   else
-    me_launch<A, false, false>(run, g);
-  run.prof_end(k);
-  ++run.launches;
+    me_launch<A, false, false>(run, g, words);
 }
 
 LARE_END  // namespace lare

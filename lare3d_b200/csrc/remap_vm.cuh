@@ -468,13 +468,17 @@ inline void vm_launch(Run<R>& run, VMArgs<R>& vm) {
   VMMaps maps;
   const long long f = 2 + 2LL * run.sx + 2LL * run.sxy;
   const auto map = [&](CUtensorMap* m, const R* p, int rows) {
-    if (!tma_map(m, p - f, run.n, run.sx, run.sxy, W, A == 1 ? 1 : rows, A == 1 ? rows : 1)) run.launch_error = true;
+    make_map(run, m, p - f, W, A == 1 ? 1 : rows, A == 1 ? rows : 1);
   };
   const R* const cells[4] = {vm.rho, vm.cv1, vm.cv2, vm.dm};
   for (int q = 0; q < 4; ++q) map(&maps.s[q], cells[q], kVmY + 1);
   map(&maps.va, g.va, kVmY + 1);
   for (int q = 0; q < 3; ++q) map(&maps.v[q], g.v[q], kVmY);
+  if (run.launch_error) return;
   const dim3 blk(32, kVmY, 1);
+  // words: v (3), v1, rho, cv1, cv2, dm read and the new v (3) written
+  const int k = run.prof_begin(A == 0 ? "remap_sweep_vert_mom_x" : "remap_sweep_vert_mom_march", 0, 11,
+                               (double)(g.nx + 1) * (g.ny + 1) * (g.nz + 1));
   if constexpr (A == 0) {
     constexpr size_t smem = VXTile<R>::smem;
     dim3 grd((g.nx + 1 + kVMXOut - 1) / kVMXOut, (g.ny + 1 + kVmY - 1) / kVmY, 1);
@@ -488,6 +492,8 @@ inline void vm_launch(Run<R>& run, VMArgs<R>& vm) {
     grd.z = (g.na + 1 + g.chunk - 1) / g.chunk;
     k_vm_march<A, R><<<grd, blk, smem, run.s>>>(maps, vm);
   }
+  run.prof_end(k);
+  ++run.launches;
 }
 
 LARE_END  // namespace lare

@@ -109,14 +109,15 @@ inline PFN_cuTensorMapEncodeTiled_v12000 tma_encoder() {
 }
 
 // The map of an array (its first element, Fortran (-2, -2, -2)) over
-// -2..n+2 with boxes of bx x by x bz.
+// -2..n+2 with boxes of bx x by x bz; false if enc (tma_encoder) is null or
+// refuses it.
 template <class R>
-inline bool tma_map(CUtensorMap* m, const R* first, const int (&n)[3], int sx, int sxy, int bx, int by, int bz) {
+inline bool tma_map(PFN_cuTensorMapEncodeTiled_v12000 enc, CUtensorMap* m, const R* first, const int (&n)[3], int sx,
+                    int sxy, int bx, int by, int bz) {
   const cuuint64_t dims[3] = {(cuuint64_t)n[0] + 5, (cuuint64_t)n[1] + 5, (cuuint64_t)n[2] + 5};
   const cuuint64_t strides[2] = {(cuuint64_t)sx * sizeof(R), (cuuint64_t)sxy * sizeof(R)};
   const cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz};
   const cuuint32_t es[3] = {1u, 1u, 1u};
-  const auto enc = tma_encoder();
   return enc && enc(m, sizeof(R) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                     const_cast<R*>(first), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
