@@ -26,6 +26,13 @@
  * no repacking.  All entry points return 0 on success and a negative
  * LARE_E* code on failure; lare_gpu_last_error() gives the message.  A
  * context is not thread-safe; it owns one CUDA stream.
+ *
+ * The step's kernels wait for their tile copies with a limit.  Where one runs
+ * out, what was computed is not to be used: from then on every call on the
+ * context that waits for the GPU and returns what kernels computed (energy,
+ * download, get_field, get_scalars, conduct_heat, conduction_stages, run, a
+ * step that returns its time or reads a count, lare_ens_sync) returns
+ * LARE_ECUDA.
  */
 #ifndef LARE_GPU_H
 #define LARE_GPU_H
@@ -398,6 +405,14 @@ int lare_gpu_check_reciprocal(const double* b, long long n, double* out, void* s
  * counterpart in the reference.
  */
 int lare_gpu_check_unmapped(int precision, long long* launches);
+
+/*
+ * Self-check of the waits for tile copies: a block waits for copies that
+ * nobody asks for.  Stores the times, in seconds, of its first wait and of a
+ * further one, and leaves the context as after a lost copy: its calls return
+ * LARE_ECUDA as described at the top.  No counterpart in the reference.
+ */
+int lare_gpu_check_lost_copy(lare_ctx* ctx, double seconds[2]);
 
 void lare_gpu_destroy(lare_ctx* ctx);
 

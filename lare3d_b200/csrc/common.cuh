@@ -176,6 +176,7 @@ enum Slot {
   SC_DTPARAB,      // explicit conduction limit
   SC_EN_B, SC_EN_KE, SC_EN_INT,
   SC_ERROR,        // LARE_E* code raised on the device (0 = none)
+  SC_LOST,         // 1 once a tile copy did not arrive (tile_wait); nothing clears or replaces it
   SC_LOOP,         // remaining resistive sub-cycles of a captured step
   SC_NSLOTS = 24
 };

@@ -194,13 +194,10 @@ __global__ void __launch_bounds__(32 * kCTY, sizeof(R) == 4 ? 5 : 2)
     mbar_init_fence();
     for (int s = -2; s < 2 && s < steps; ++s) issue(s);
   }
-  bool dead = false;  // a copy never arrived: flagged, and no more waiting
+  int dead = 0;
   auto await = [&](int s) {
     const int q = s + 2;
-    if (!dead && !mbar_wait(bar_s + 8 * (q % kStT), (uint32_t)(q / kStT) & 1u)) {
-      dead = true;
-      a.sc[SC_ERROR] = (double)LARE_ECUDA;
-    }
+    tile_wait(bar_s + 8 * (q % kStT), (uint32_t)(q / kStT) & 1u, dead, a.sc);
   };
   const R tc = a.tc, te0 = a.te0, k0 = a.k0;
   const R dt = (R)a.sc[a.dt_slot];

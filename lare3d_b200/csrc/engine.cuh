@@ -897,11 +897,22 @@ void eulerian_remap(Run<R>& run, int step) {
   // bfield_bcs at remap.f90:128 would write the same values again)
 }
 
+// LARE_ECUDA, with its message, where the scalar slots on the host say that a
+// kernel's tile copy was lost: what it computed is not to be used.
+template <class R>
+int lost_copy(Run<R>& run) {
+  if (run.host_sc[SC_LOST] == 0.0) return LARE_OK;
+  run.err = "a tile copy never arrived";
+  return LARE_ECUDA;
+}
 // Pull the scalar slots to the host (one sync).
 template <class R>
-cudaError_t pull_scalars(Run<R>& run) {
+int pull_scalars(Run<R>& run) {
   cudaMemcpyAsync(run.host_sc, run.sc, SC_NSLOTS * sizeof(double), cudaMemcpyDeviceToHost, run.s);
-  return cudaStreamSynchronize(run.s);
+  const cudaError_t e = cudaStreamSynchronize(run.s);
+  if (e == cudaSuccess) return lost_copy(run);
+  run.err = std::string("sync failed: ") + cudaGetErrorString(e);
+  return LARE_ECUDA;
 }
 
 // ---------------------------------------------------------------------

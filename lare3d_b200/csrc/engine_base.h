@@ -41,6 +41,7 @@ class EngineBase {
   virtual void add_steps(int n) = 0;
   virtual int set_block(int bx, int by) = 0;
   virtual int device_error() = 0;  // syncs; LARE_E* raised on the device, 0 if none
+  virtual int check_lost_copy(double seconds[2]) = 0;
   virtual long long launches() const = 0;
   virtual void* stream() const = 0;
   virtual const char* error() const = 0;

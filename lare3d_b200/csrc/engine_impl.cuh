@@ -60,6 +60,28 @@ __global__ void k_fill(R* p, size_t n, R v) {
   if (t < n) p[t] = v;
 }
 
+// A block whose warps wait, as the kernels' do, for copies that nobody asks for:
+// ns[0] is the time of the first wait, ns[1] of one after it.
+template <class R>
+__global__ void k_lost_copy(double* sc, double* ns) {
+  __shared__ __align__(8) unsigned long long bar;
+  const uint32_t b = smem_addr(&bar);
+  if (threadIdx.x == 0) {
+    mbar_init(b, 1);
+    mbar_init_fence();
+  }
+  __syncthreads();
+  int dead = 0;
+  for (int q = 0; q < 2; ++q) {
+    unsigned long long t0, t1;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    tile_wait(b, 0u, dead, sc);
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
+    if (threadIdx.x == 0) ns[q] = (double)(t1 - t0);
+    __syncthreads();
+  }
+}
+
 template <class R>
 class EngineT : public EngineBase {
  public:
@@ -87,6 +109,16 @@ class EngineT : public EngineBase {
     if (e != cudaSuccess) return fail(LARE_ECUDA, std::string(where) + ": " + cudaGetErrorString(e));
     if (run.launch_error) return fail(LARE_ECUDA, std::string(where) + ": tensor map");
     return LARE_OK;
+  }
+
+  // the scalar slots to the host, for a call that waits for the GPU
+  int pull(const char* where) {
+    const int rc = pull_scalars(run);
+    return rc ? fail(rc, std::string(where) + ": " + run.err) : LARE_OK;
+  }
+  // the status of the kernels so far, for lost_copy after the wait to come
+  void status_along() {
+    cudaMemcpyAsync(run.host_sc + SC_LOST, run.sc + SC_LOST, sizeof(double), cudaMemcpyDeviceToHost, run.s);
   }
 
   template <class T>
@@ -492,7 +524,9 @@ class EngineT : public EngineBase {
   }
 
   int lagrangian_step(int step) override {
+    run.err.clear();
     int rc = lare::lagrangian_step(run, step);
+    if (rc == LARE_ECUDA && !run.err.empty()) return fail(rc, "lagrangian_step: " + run.err);
     if (rc) return fail(rc, rc == LARE_EDT ? "dt underflow or non-finite dt" : "lagrangian_step failed");
     if (run.pip) {
       if ((rc = eos_error())) return rc;
@@ -501,7 +535,7 @@ class EngineT : public EngineBase {
   }
   // LARE_EEOS raised by a neutral_fraction launch (syncs)
   int eos_error() {
-    if (pull_scalars(run) != cudaSuccess) return fail(LARE_ECUDA, "sync failed");
+    if (const int rc = pull("neutral_fraction")) return rc;
     if ((int)run.host_sc[SC_ERROR] == LARE_EEOS)
       return fail(LARE_EEOS, "neutral_fraction: temperature bounds problem (empty bracket)");
     return LARE_OK;
@@ -541,7 +575,7 @@ class EngineT : public EngineBase {
     if (rc) return rc;
     cudaMemcpyAsync(run.sc + SC_DTCOND, &dt, sizeof(double), cudaMemcpyHostToDevice, run.s);
     calc_s_stages(run, SC_DTCOND);
-    if (pull_scalars(run) != cudaSuccess) return fail(LARE_ECUDA, "conduct_heat: sync failed");
+    if (const int rc = pull("conduct_heat")) return rc;
     int ns = force_stages > 0 ? force_stages : (int)run.host_sc[SC_STAGES];
     if (ns < 1 || ns > 100000) return fail(LARE_ESTAGES, "RKL2 stage count out of range");
     run.n_s_stages = ns;
@@ -551,7 +585,7 @@ class EngineT : public EngineBase {
   }
   int energy(double out[5]) override {
     energy_account(run);
-    if (pull_scalars(run) != cudaSuccess) return fail(LARE_ECUDA, "energy: sync failed");
+    if (const int rc = pull("energy")) return rc;
     out[0] = run.host_sc[SC_EN_B];
     out[1] = run.host_sc[SC_EN_KE];
     out[2] = run.host_sc[SC_EN_INT];
@@ -561,18 +595,21 @@ class EngineT : public EngineBase {
   }
   int download(double* const* s8) override {
     static const char* names[8] = {"rho", "energy", "vx", "vy", "vz", "bx", "by", "bz"};
+    status_along();
     for (int q = 0; q < 8; ++q) {
       if (!s8[q]) continue;
       auto& f = fields[names[q]];
       int rc = get(*f.first, f.second, s8[q]);
       if (rc) return rc;
     }
-    return LARE_OK;
+    return lost_copy(run);
   }
   int get_field(const char* name, double* host) override {
     auto it = fields.find(name);
     if (it == fields.end()) return fail(LARE_ENOTFOUND, std::string("unknown field ") + name);
-    return get(*it->second.first, it->second.second, host);
+    status_along();
+    const int rc = get(*it->second.first, it->second.second, host);
+    return rc ? rc : lost_copy(run);
   }
   int set_field(const char* name, const double* host) override {
     auto it = fields.find(name);
@@ -617,6 +654,15 @@ class EngineT : public EngineBase {
     return cuda_check("capture_steps");
   }
   void add_steps(int n) override { run.steps_taken += n; }
+  int check_lost_copy(double seconds[2]) override {
+    k_lost_copy<R><<<1, 256, 0, run.s>>>(run.sc, staging);
+    double ns[2] = {0.0, 0.0};
+    cudaMemcpyAsync(ns, staging, sizeof(ns), cudaMemcpyDeviceToHost, run.s);
+    cudaError_t e = cudaStreamSynchronize(run.s);
+    if (e != cudaSuccess) return fail(LARE_ECUDA, cudaGetErrorString(e));
+    for (int q = 0; q < 2; ++q) seconds[q] = 1e-9 * ns[q];
+    return LARE_OK;
+  }
   int set_block(int bx, int by) override {
     if (bx < 1 || by < 1 || bx * by > 256 || (bx * by) % 32) return fail(LARE_EINVAL, "block shape");
     run.blk_x = bx;
@@ -624,7 +670,7 @@ class EngineT : public EngineBase {
     return LARE_OK;
   }
   int device_error() override {
-    if (pull_scalars(run) != cudaSuccess) return fail(LARE_ECUDA, "device_error: sync failed");
+    if (const int rc = pull("device_error")) return rc;
     const int code = (int)run.host_sc[SC_ERROR];
     if (code) fail(code, "raised on the device in a recorded step (bad dt, sub-cycle count or EOS bracket)");
     return code;
@@ -634,7 +680,7 @@ class EngineT : public EngineBase {
     if (rc) return rc;
     cudaMemcpyAsync(run.sc + SC_DTCOND, &dt, sizeof(double), cudaMemcpyHostToDevice, run.s);
     calc_s_stages(run, SC_DTCOND);
-    if (pull_scalars(run) != cudaSuccess) return fail(LARE_ECUDA, "conduction_stages: sync failed");
+    if (const int rc = pull("conduction_stages")) return rc;
     *n_stages = (int)run.host_sc[SC_STAGES];
     return cuda_check("conduction_stages");
   }
@@ -652,8 +698,7 @@ class EngineT : public EngineBase {
     return LARE_OK;
   }
   int scalars(lare_scalars* o) override {
-    if (pull_scalars(run) != cudaSuccess) return fail(LARE_ECUDA, "scalars: sync failed");
-    if ((int)run.host_sc[SC_ERROR] == LARE_ECUDA) return fail(LARE_ECUDA, "a tile copy never arrived");
+    if (const int rc = pull("scalars")) return rc;
     o->time = run.host_sc[SC_TIME];
     o->dt = run.host_sc[SC_DT];
     o->dtr = run.host_sc[SC_DTR];

@@ -1097,7 +1097,7 @@ int lagrangian_step(Run<R>& run, int step) {
     int rc = resistive_subcycles_captured(run);
     if (rc) return rc;
   } else if (run.p.resistive_mhd) {
-    if (pull_scalars(run) != cudaSuccess) return LARE_ECUDA;
+    if (const int rc = pull_scalars(run)) return rc;
     int substeps = (int)run.host_sc[SC_SUBSTEPS];
     double dtv = run.host_sc[SC_DT];
     if (!(dtv > 0.0) || !std::isfinite(dtv)) return LARE_EDT;
@@ -1115,7 +1115,7 @@ int lagrangian_step(Run<R>& run, int step) {
     if (run.capturing) return LARE_EINVAL;  // the stage count and coefficients are host-side
     copy_whole(run, run.a.energy0, run.a.energy);
     calc_s_stages(run, SC_DT);
-    if (pull_scalars(run) != cudaSuccess) return LARE_ECUDA;
+    if (const int rc = pull_scalars(run)) return rc;
     int ns = (int)run.host_sc[SC_STAGES];
     if (ns < 1 || ns > 100000) return LARE_ESTAGES;
     run.n_s_stages = ns;

@@ -265,6 +265,11 @@ int lare_gpu_check_unmapped(int precision, long long* launches) {
   return LARE_EINVAL;
 }
 
+int lare_gpu_check_lost_copy(lare_ctx* c, double seconds[2]) {
+  if (guard(c) || !seconds) return LARE_EINVAL;
+  return c->e->check_lost_copy(seconds);
+}
+
 void* lare_gpu_stream(lare_ctx* c) { return (c && c->e) ? c->e->stream() : nullptr; }
 
 const char* lare_gpu_last_error(lare_ctx* c) {

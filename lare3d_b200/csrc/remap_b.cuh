@@ -284,13 +284,8 @@ __global__ void __launch_bounds__(32 * kBsY, sizeof(R) == 8 ? 2 : 3) k_bsweep_ma
   };
   BWin<R> w1, w2;
   R db0, dbp;
-  bool dead = false;  // a copy never arrived: flagged, and no more waiting
-  auto await = [&](int slot, uint32_t parity) {
-    if (!dead && !mbar_wait(bar_s + 8 * slot, parity)) {
-      dead = true;
-      g.sc[SC_ERROR] = (double)LARE_ECUDA;
-    }
-  };
+  int dead = 0;
+  auto await = [&](int slot, uint32_t parity) { tile_wait(bar_s + 8 * slot, parity, dead, g.sc); };
   __syncthreads();  // the barriers are set up
   {
     // windows of the first flux; the stencil is clamped as MAX(ia-1, -1)
@@ -470,13 +465,8 @@ __global__ void __launch_bounds__(32 * kBsY, sizeof(R) == 8 ? 2 : 4) k_bsweep_x(
   // db1 from the face velocity of this lane's x and the one below
   auto width = [&](R vf) { return mx + (vf - __shfl_up_sync(all, vf, 1)) * dt; };
   auto face = [&](R a, R b, R c, R d) { return (a + b + c + d) * q4; };
-  bool dead = false;  // a copy never arrived: flagged, and no more waiting
-  auto await = [&](int slot, uint32_t parity) {
-    if (!dead && !mbar_wait(bar_s + 8 * slot, parity)) {
-      dead = true;
-      g.sc[SC_ERROR] = (double)LARE_ECUDA;
-    }
-  };
+  int dead = 0;
+  auto await = [&](int slot, uint32_t parity) { tile_wait(bar_s + 8 * slot, parity, dead, g.sc); };
   __syncthreads();  // the barriers are set up
   await(0, 0);
   await(1, 0);

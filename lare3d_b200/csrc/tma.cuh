@@ -43,13 +43,21 @@ __device__ __forceinline__ bool mbar_done(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Wait for a phase, at most kMbarSpins tries (each suspends the thread for a
+// Wait for a phase, at most kMbarTries tries (each suspends the thread for a
 // while in hardware); false if it never completed.
-constexpr int kMbarSpins = 1 << 20;
+constexpr int kMbarTries = 1 << 20;
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  for (int i = 0; i < kMbarSpins; ++i)
+  for (int i = 0; i < kMbarTries; ++i)
     if (mbar_done(bar, parity)) return true;
   return false;
+}
+// A kernel's wait for a tile copy.  One that runs out raises SC_LOST in sc and
+// marks the thread `dead`: it waits no more.
+__device__ __forceinline__ void tile_wait(uint32_t bar, uint32_t parity, int& dead, double* sc) {
+  if (!dead && !mbar_wait(bar, parity)) {
+    dead = 1;
+    sc[SC_LOST] = 1.0;
+  }
 }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2,
                                             uint32_t bar) {
@@ -62,15 +70,12 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
 
 // A ring of NS shared-memory slots filled by one thread and read by all warps
 // of a block: a full barrier a slot counts the bytes of its copies, an empty
-// one the warps that are done with it.  Step k uses slot k % NS.  A wait that
-// runs out (a copy that never arrives) raises LARE_ECUDA in sc and is not
-// repeated, so that the block still ends.
+// one the warps that are done with it.  Step k uses slot k % NS.
 template <int NS>
 struct TileRing {
   uint32_t full, empty, base;  // shared-memory addresses: barriers, slot 0
-  int bytes;                   // a slot
   double* sc;
-  bool dead = false;
+  int dead = 0;
   // one thread, before a block barrier
   __device__ __forceinline__ void init(int warps) {
     for (int s = 0; s < NS; ++s) {
@@ -80,10 +85,7 @@ struct TileRing {
     mbar_init_fence();
   }
   __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity) {
-    if (!dead && !mbar_wait(bar, parity)) {
-      dead = true;
-      sc[SC_ERROR] = (double)LARE_ECUDA;
-    }
+    tile_wait(bar, parity, dead, sc);
   }
   __device__ __forceinline__ void wait_full(int slot, uint32_t parity) { wait(full + 8 * slot, parity); }
   // a warp is done with a slot
