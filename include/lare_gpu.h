@@ -408,8 +408,9 @@ int lare_gpu_check_unmapped(int precision, long long* launches);
 
 /*
  * Self-check of the waits for tile copies: a block waits for copies that
- * nobody asks for.  Stores the times, in seconds, of its first wait and of a
- * further one, and leaves the context as after a lost copy: its calls return
+ * nobody asks for.  Stores the times, in seconds, of its first wait (which
+ * has to end by itself after about a second) and of a further one (which is
+ * left out), and leaves the context as after a lost copy: its calls return
  * LARE_ECUDA as described at the top.  No counterpart in the reference.
  */
 int lare_gpu_check_lost_copy(lare_ctx* ctx, double seconds[2]);

@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(32 * kCTY, sizeof(R) == 4 ? 5 : 2)
     if (s + 1 < steps) own1 = convert(s + 1);
     __syncthreads();
     // every thread is past the last step: its slots are free
-    if (boss && s + 2 < steps) {
+    if (boss && !dead && s + 2 < steps) {
       // the copy overwrites a plane that threads wrote (converted) before the barrier
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       issue(s + 2);

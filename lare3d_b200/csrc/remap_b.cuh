@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(32 * kBsY, sizeof(R) == 8 ? 2 : 3) k_bsweep_ma
     const R f1b = __shfl_up_sync(0xffffffffu, f1, 1);
     __syncthreads();
     // every thread is past the last step: the slots of the planes below ia are free
-    if (boss)
+    if (boss && !dead)
       for (; next <= pe && next < ia + kBsStages; ++next) issue(next, (next - p0) % kBsStages);
     if (wr && ia >= o0) {
       R b1 = b[0], b2 = b[L::b / (int)sizeof(R)], bA = b[2 * L::b / (int)sizeof(R)];
@@ -514,7 +514,7 @@ __global__ void __launch_bounds__(32 * kBsY, sizeof(R) == 8 ? 2 : 4) k_bsweep_x(
     const R f1l = __shfl_up_sync(all, f1, 1), f2l = __shfl_up_sync(all, f2, 1);
     __syncthreads();
     // every thread is past the last step: the slots of the planes below iz are free
-    if (boss)
+    if (boss && !dead)
       for (; next <= pe && next < iz + kBsStages; ++next) issue(next, (next - p0) % kBsStages);
     if (wr && iz >= o0) {
       const R* const b = reinterpret_cast<const R*>(ring + s0 * L::slot + L::va) + cb;

@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(32 * kMeY, sizeof(R) == 8 ? 2 : 4)
     if (boss && ia > first && ia - 1 + kMeSlots <= ia1) {
       const int ps = slot == 0 ? kMeSlots - 1 : slot - 1;
       ring.wait(ring.empty + 8 * ps, slot == 0 ? ph ^ 1u : ph);
-      issue(ia - 1 + kMeSlots, ps);
+      if (!ring.dead) issue(ia - 1 + kMeSlots, ps);
     }
     if (++slot == kMeSlots) {
       slot = 0;
@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(32 * kMeY, sizeof(R) == 8 ? 2 : 4)
     if (boss && iz > iz0 && iz - 1 + kMeSlots <= iz1) {
       const int ps = slot == 0 ? kMeSlots - 1 : slot - 1;
       ring.wait(ring.empty + 8 * ps, slot == 0 ? ph ^ 1u : ph);
-      issue(iz - 1 + kMeSlots, ps);
+      if (!ring.dead) issue(iz - 1 + kMeSlots, ps);
     }
     if (++slot == kMeSlots) {
       slot = 0;

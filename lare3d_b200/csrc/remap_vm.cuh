@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(32 * kVmY, sizeof(R) == 8 ? 2 : 3)
     if (boss && ia > ia0 && ia - 1 + kVmSlots <= ia1) {
       const int ps = slot == 0 ? kVmSlots - 1 : slot - 1;
       ring.wait(ring.empty + 8 * ps, slot == 0 ? ph ^ 1u : ph);
-      issue(ia - 1 + kVmSlots, ps);
+      if (!ring.dead) issue(ia - 1 + kVmSlots, ps);
     }
     if (++slot == kVmSlots) {
       slot = 0;
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(32 * kVmY, sizeof(R) == 8 ? 2 : 3)
     if (boss && iz > iz0 && iz - 1 + kVmSlots <= iz1) {
       const int ps = slot == 0 ? kVmSlots - 1 : slot - 1;
       ring.wait(ring.empty + 8 * ps, slot == 0 ? ph ^ 1u : ph);
-      issue(iz - 1 + kVmSlots, ps);
+      if (!ring.dead) issue(iz - 1 + kVmSlots, ps);
     }
     if (++slot == kVmSlots) {
       slot = 0;

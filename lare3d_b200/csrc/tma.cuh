@@ -43,21 +43,26 @@ __device__ __forceinline__ bool mbar_done(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Wait for a phase, at most kMbarTries tries (each suspends the thread for a
-// while in hardware); false if it never completed.
-constexpr int kMbarTries = 1 << 20;
+// Wait for a phase, for about a second (a try that fails suspends the thread
+// for 4 us on a B200); false if it never completed.
+constexpr int kMbarTries = 1 << 18;
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   for (int i = 0; i < kMbarTries; ++i)
     if (mbar_done(bar, parity)) return true;
   return false;
 }
 // A kernel's wait for a tile copy.  One that runs out raises SC_LOST in sc and
-// marks the thread `dead`: it waits no more.
+// marks the thread `dead`: it waits no more, and a dead thread asks for no more
+// copies, so that the block ends with every copy that it asked for a second or
+// more in the past.
 __device__ __forceinline__ void tile_wait(uint32_t bar, uint32_t parity, int& dead, double* sc) {
   if (!dead && !mbar_wait(bar, parity)) {
     dead = 1;
     sc[SC_LOST] = 1.0;
   }
+  // (opaque: told apart by `dead`, the marching loops were compiled twice over,
+  // and the mass/energy and momentum sweeps took 10 % longer at 256^3)
+  asm volatile("" : "+r"(dead));
 }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2,
                                             uint32_t bar) {
