@@ -619,8 +619,8 @@ void set_dt(Run<R>& run) {
 template <class R>
 void predictor_remap(Run<R>& run, int step) {
   Arrays<R>& A = run.a;
-  // The sweeps carry B from the step's arrays through the B0 and B1 buffers
-  // (the first puts it in flux form, the last back: remap.f90:43-69, :101-127),
+  // The sweeps carry B from the step's arrays through the B0 buffers and three
+  // that the corrector's remap fills later (the first puts it in flux form, the last back: remap.f90:43-69, :101-127),
   // so B itself is kept as B0.  vx1 = vx (lagran.F90:1051-1053): the sweeps
   // read v itself.  vx1's own nodes 0:n are rewritten by the predictor force
   // and its ghosts by remap_v_bcs, except on an open side: there the copy's
@@ -630,7 +630,7 @@ void predictor_remap(Run<R>& run, int step) {
   carry_velocity(run, keep, v);
   R* const b[3] = {A.bx.p, A.by.p, A.bz.p};
   R* const p[3] = {A.bx0.p, A.by0.p, A.bz0.p};
-  R* const q[3] = {A.bx1.p, A.by1.p, A.bz1.p};
+  R* const q[3] = {A.cv2.p, A.dm.p, A.flux.p};
   const int* const order = sweep_order(step);
   for (int s = 0; s < 3; ++s) {
     const int bmode = s == 0 ? 1 : (s == 2 ? 2 : 0);

@@ -436,14 +436,15 @@ void remap_sweep(Run<R>& run, int dt_slot, int pass[3], int bmode) {
   const R pass_t1 = (R)pass[T1], pass_t2 = (R)pass[T2];
   const double* sc = run.sc;
 
-  // ---- K1: B, into the second set of arrays
+  // ---- K1: B, into the arrays of the Lagrangian step's B0, whose work is done
+  // (bx1, by1, bz1 are named fields: the B before the last resistive sub-cycle)
   {
     R* const in[3] = {Ar.bx.p, Ar.by.p, Ar.bz.p};
-    R* const out[3] = {Ar.bx1.p, Ar.by1.p, Ar.bz1.p};
+    R* const out[3] = {Ar.bx0.p, Ar.by0.p, Ar.bz0.p};
     bsweep<A>(run, va, in, out, dt_slot, bmode);
-    std::swap(Ar.bx.p, Ar.bx1.p);
-    std::swap(Ar.by.p, Ar.by1.p);
-    std::swap(Ar.bz.p, Ar.bz1.p);
+    std::swap(Ar.bx.p, Ar.bx0.p);
+    std::swap(Ar.by.p, Ar.by0.p);
+    std::swap(Ar.bz.p, Ar.bz0.p);
   }
 
   R* const rho = Ar.rho.p;        // rho1 of the reference from here on
