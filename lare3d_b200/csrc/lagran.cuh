@@ -533,9 +533,9 @@ void set_dt(Run<R>& run) {
       // and outside the range that the estimate can judge, and the minima are
       // the same bit for bit.  In FP32 the pass over memory bounds.
       const R b1 = (R)best[0], b3 = (R)best[1], slack = R(0.9995);
-      const float s = (float)(gp + gb * w1 + pv), q = (float)rho0, b = (float)best[0];
-      const float own = (float)length * sqrtf(q) * 0.998f, lim = b * (sqrtf((float)pv) + sqrtf(s));
-      bool out = own > lim && own > 1e-30f && own < 1e30f && s > 1e-28f && q > 1e-30f && q < 1e30f && b > 1e-30f && b < 1e30f;
+      const float s = (float)(gp + gb * w1 + pv), q = (float)rho0, b = (float)best[0], l = (float)length;
+      const float own = l * sqrtf(q) * 0.998f, lim = b * (sqrtf((float)pv) + sqrtf(s));
+      bool out = own > lim && l > 1e-30f && own > 1e-30f && own < 1e30f && s > 1e-28f && q > 1e-30f && q < 1e30f && b > 1e-30f && b < 1e30f;
       out = out && hx * slack > b1 * ux && hy * slack > b1 * uy && hz * slack > b1 * uz;
       if (out && (cowling || resistive)) {
         const R hx2 = hx * hx, hy2 = hy * hy, hz2 = hz * hz;
