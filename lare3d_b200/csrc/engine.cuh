@@ -332,14 +332,18 @@ inline void box_min(Run<R>& run, const char* site, int i0, int i1, int j0, int j
                     int words = 0) {
   int ni = i1 - i0 + 1, nj = j1 - j0 + 1, nk = k1 - k0 + 1;
   // planes per block: fewer blocks contend for the atomic, and later blocks
-  // find lower minima recorded (set_dt leaves out most cells by them).  At
-  // 256^3 in FP64 1 plane takes 0.52 ms for set_dt, 4 0.41, 8 0.35 and 12
-  // 0.35; at 80^3 8 take 29 us and 12 34.  FP32: 0.23 -> 0.18 ms from 1 to 8.
-  constexpr int kMinPlanes = 8;
+  // find lower minima recorded (set_dt leaves out most cells by them), but a
+  // thread takes its planes one after another, so a grid that has less than
+  // five blocks an SM takes fewer.  set_dt in FP64 with 1, 2, 4 and 8 planes:
+  // 12^3 8.6, 10, 13 and 17 us; 64^3 21, 18, 17 and 21; 96^3 42, 37, 39 and
+  // 44; 128^3 87, 74, 70 and 69; 256^3 507, 417, 373 and 353.
   dim3 blk(64, 4, 1);
-  dim3 grd((ni + 63) / 64, (nj + 3) / 4, (nk + kMinPlanes - 1) / kMinPlanes);
+  dim3 grd((ni + 63) / 64, (nj + 3) / 4, 1);
+  int planes = 8;
+  while (planes > 1 && (long long)grd.x * grd.y * ((nk + planes - 1) / planes) < 5 * 148) planes /= 2;
+  grd.z = (nk + planes - 1) / planes;
   int k = run.prof_begin(site, 0, words, (double)ni * nj * nk);
-  k_box_min<NV><<<grd, blk, 0, run.s>>>(i0, j0, k0, ni, nj, nk, kMinPlanes, fn, run.us + uslot);
+  k_box_min<NV><<<grd, blk, 0, run.s>>>(i0, j0, k0, ni, nj, nk, planes, fn, run.us + uslot);
   run.prof_end(k);
   ++run.launches;
 }
