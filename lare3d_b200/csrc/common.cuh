@@ -34,7 +34,7 @@ struct A1 {
 // Elements by their byte offset from an array's first element, Fortran
 // (-2, -2, -2).  All arrays share one layout, so one 32-bit offset serves
 // every array at a point, where an element index costs a 64-bit multiply-add
-// per array.  It cannot overflow: a context holds more than 50 arrays, so on
+// per array.  It cannot overflow: a context holds 50 arrays or more, so on
 // a GPU of less than 200 GB one array stays below 2^32 bytes.
 template <class R>
 __device__ __forceinline__ unsigned elem_off(int i, int si, int j, int sj) {

@@ -54,10 +54,8 @@ struct Arrays {
   // lagran.F90 temporaries
   A3<R> bx0, by0, bz0, bx1, by1, bz1, alpha1, alpha2, alpha3, visc_heat, pressure, rho_v, cv_v;
   A3<R> flux_x, flux_y, flux_z, curlb, fx_visc, fy_visc, fz_visc, qx, qy, qz, energy0, cs, cs_v;
-  // [xyz]remap.f90 temporaries (f1, f2: the two B fluxes; rho_alt: second
-  // density buffer; cv1v, cv2v, dmv: vertex averages; mf?: momentum fluxes)
-  A3<R> db1, dc1, r_rho_v, r_rho_v1, rho1, dm, cv2, flux;
-  A3<R> f1, f2, rho_alt, cv1v, cv2v, dmv, mfx, mfy, mfz;
+  // [xyz]remap.f90 temporaries (rho_alt, flux: second buffers of density and energy)
+  A3<R> dm, cv2, flux, rho_alt;
   // conduct.f90 temporaries
   A3<R> larsen, Y1, Y2, Y3, Lc_Y0;  // RKL2 (Y0 is read from energy itself)
   A3<R> kf[9];                        // stage-invariant face coefficients, 3 per face direction
@@ -65,9 +63,11 @@ struct Arrays {
   A3<R> xi, eta_perp;
   // the energy after rad_losses (radiative.f90), allocated with radiation on
   A3<R> erad;
-  // rke: the remap's kinetic-energy defect (shared_data.F90:108) and the
-  // three momentum fluxes before their product with dm
+  // rke: the remap's kinetic-energy defect (shared_data.F90:108), the three
+  // momentum fluxes before their product with dm, and what the split momentum
+  // kernels read: the moved widths and the vertex averages
   A3<R> delta_ke, rke_f[3], rke_dk[3];
+  A3<R> db1, dc1, r_rho_v, r_rho_v1, cv1v, cv2v, dmv;
   // cooling_term: moving averages of the viscous and ohmic heating
   // (shared_data.F90:109), persistent across steps
   A3<R> cool_term_v, cool_term_b;
@@ -457,7 +457,7 @@ inline int resident_blocks(int threads, size_t smem = 0) {
 // the GPU at once: the number of chunks that makes the fewest steps, a wave of
 // blocks taking a chunk's points and about kMarchStart steps to fill its
 // windows.  So a large grid gets long chunks (up to cap), a small one as many
-// as run at once, down to 4 points, and no last wave is left nearly empty.
+// as run at once, down to 3 or 4 points, and no last wave is left nearly empty.
 // With fixed chunks of 16 and 32 a 64^3 grid left most SMs idle (the march of
 // eta_calc took 52 us on 96 x 80 x 121 with 8 % of the resident blocks).
 constexpr int kMarchStart = 4;
@@ -824,13 +824,10 @@ __device__ __forceinline__ LimOut<R> limiter_dv(R v_advect, R fm, R fi, R fp, R 
 // above c): the reference's expressions regrouped, with the upwind choices
 // (whose weights are exactly 0 or 1) and the product of signs taken by
 // selection.  phi = |v dt| * rxu; the result is (f_u + D (1 - phi)) v dt.
+// (kRegroup only, so in FP64.)
 template <class R>
 __device__ __forceinline__ R lesser(R a, R b) {
   return a < b ? a : b;
-}
-template <>
-__device__ __forceinline__ float lesser(float a, float b) {
-  return fminf(a, b);
 }
 // copies +-m: zero unless a and b have the same sign, else m with the sign of a * s
 __device__ __forceinline__ double signed_min(double m, double a, double b, double s) {
@@ -838,11 +835,6 @@ __device__ __forceinline__ double signed_min(double m, double a, double b, doubl
   const bool same = (ha ^ __double2hiint(b)) >= 0;
   const int h = __double2hiint(m) | ((ha ^ __double2hiint(s)) & 0x80000000);
   return same ? __hiloint2double(h, __double2loint(m)) : 0.0;
-}
-__device__ __forceinline__ float signed_min(float m, float a, float b, float s) {
-  const int ha = __float_as_int(a);
-  const bool same = (ha ^ __float_as_int(b)) >= 0;
-  return same ? __int_as_float(__float_as_int(m) | ((ha ^ __float_as_int(s)) & 0x80000000)) : 0.0f;
 }
 template <class R>
 __device__ __forceinline__ R van_leer(R v, R vdt, R f0, R fp, R dm, R d0, R dp, R sm, R s0, R sp, R db0, R dbp, R r0,

@@ -223,7 +223,7 @@ class EngineT : public EngineBase {
     long long elems = sxy * sz;
     if (elems >= (1LL << 31)) { err = "grid too large for 32-bit indexing"; return LARE_EINVAL; }
     // byte offsets within an array are 32-bit (elem_at): an array past that
-    // is one of more than 50, which no GPU of less than 200 GB holds
+    // is one of 50 or more, which no GPU of less than 200 GB holds
     if (elems * (long long)sizeof(R) >= (1LL << 32)) { err = "cudaMalloc: an array of 4 GiB or more"; return LARE_ENOMEM; }
     run.sxy = (int)sxy;
     run.elems = (size_t)elems;
@@ -247,9 +247,8 @@ class EngineT : public EngineBase {
         &run.a.bz0, &run.a.bx1, &run.a.by1, &run.a.bz1, &run.a.alpha1, &run.a.alpha2, &run.a.alpha3,
         &run.a.visc_heat, &run.a.pressure, &run.a.rho_v, &run.a.cv_v, &run.a.flux_x, &run.a.flux_y,
         &run.a.flux_z, &run.a.curlb, &run.a.fx_visc, &run.a.fy_visc, &run.a.fz_visc, &run.a.qx, &run.a.qy,
-        &run.a.qz, &run.a.energy0, &run.a.cs, &run.a.cs_v, &run.a.db1, &run.a.dc1, &run.a.r_rho_v,
-        &run.a.r_rho_v1, &run.a.rho1, &run.a.dm, &run.a.cv2, &run.a.flux, &run.a.f1, &run.a.f2,
-        &run.a.rho_alt, &run.a.cv1v, &run.a.cv2v, &run.a.dmv, &run.a.mfx, &run.a.mfy, &run.a.mfz};
+        &run.a.qz, &run.a.energy0, &run.a.cs, &run.a.cs_v, &run.a.dm, &run.a.cv2, &run.a.flux,
+        &run.a.rho_alt};
     if (p.conduction) {
       for (A3<R>* x : {&run.a.larsen, &run.a.Y1, &run.a.Y2, &run.a.Y3, &run.a.Lc_Y0})
         all.push_back(x);
@@ -262,7 +261,8 @@ class EngineT : public EngineBase {
     if (p.radiation) all.push_back(&run.a.erad);
     if (p.rke)
       for (A3<R>* x : {&run.a.delta_ke, &run.a.rke_f[0], &run.a.rke_f[1], &run.a.rke_f[2], &run.a.rke_dk[0],
-                       &run.a.rke_dk[1], &run.a.rke_dk[2]})
+                       &run.a.rke_dk[1], &run.a.rke_dk[2], &run.a.db1, &run.a.dc1, &run.a.r_rho_v,
+                       &run.a.r_rho_v1, &run.a.cv1v, &run.a.cv2v, &run.a.dmv})
         all.push_back(x);
     if (p.cooling_term)
       for (A3<R>* x : {&run.a.cool_term_v, &run.a.cool_term_b}) all.push_back(x);

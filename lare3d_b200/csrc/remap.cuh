@@ -15,10 +15,11 @@
 //                 into a second buffer (old rho stays readable as rho1), the
 //                 energy flux (:539-601) and the new energy (:187-196)
 //                 (remap_me.cuh).
-//   K7 vertex     vertex rho_v, cv1, cv2, dm averages and rho_v1 (:201-290).
+//   K7 vertex     vertex rho_v, cv1, cv2, dm averages and rho_v1 (:201-290),
 //   K8 momentum   the three momentum fluxes (:605-895), each times dm, and
-//   K9 velocity   the three velocity updates (:292-329), fused into one
-//                 kernel that writes the new velocities to second buffers.
+//   K9 velocity   the three velocity updates (:292-329), one kernel that
+//                 writes the new velocities to second buffers (remap_vm.cuh);
+//                 with rke on K7 is a kernel of its own (below).
 // The face-averaged vx1 written back at :265 is only read again as
 // REAL(xpass)*(...) with xpass = 0, so it is formed in K8 and not stored.
 // The predictor's sweeps (predictor_step = .TRUE.) are K1 alone.
@@ -182,7 +183,7 @@ struct MomArgs {
   const R* cv1v;
   const R* cv2v;
   const R* rv1;
-  R* fp[3];  // rke only: the fluxes before their product with dm
+  R* fp[3];  // rke: the fluxes before their product with dm
   A1<R> dct1, dct2;
   double* sc;
   int dt_slot, nx, ny, nz, na, n3, sx, sxy, SA, S3;
@@ -257,9 +258,9 @@ __device__ __forceinline__ void mom_flux_vals(R area, R va0, R va1, R rvc, R rvp
   }
 }
 
-// the same, loading the stencil of face c (RKE: also store the fluxes
-// before their product with dm in g.fp)
-template <class R, bool RKE = false>
+// the same, loading the stencil of face c and storing the fluxes before their
+// product with dm in g.fp
+template <class R>
 __device__ __forceinline__ void mom_flux(const MomArgs<R>& g, int c, int i1, int i2, R dt, R (&F)[3]) {
   const int SA = g.SA;
   R w[3][4];
@@ -268,12 +269,10 @@ __device__ __forceinline__ void mom_flux(const MomArgs<R>& g, int c, int i1, int
 #pragma unroll
     for (int q = 0; q < 4; ++q) w[comp][q] = g.v[comp][c + (q - 1) * SA];
   R fpre[3];
-  mom_flux_vals<R, RKE>(g.dct1(i1) * g.dct2(i2), g.va[c], g.va[c + SA], g.rv[c], g.rv[c + SA], g.dmv[c],
-                               g.db1[c], g.db1[c + SA], g.db1[c + 2 * SA], g.dc1[c], g.dc1[c + SA], w, dt, F, fpre);
-  if constexpr (RKE) {
+  mom_flux_vals<R, true>(g.dct1(i1) * g.dct2(i2), g.va[c], g.va[c + SA], g.rv[c], g.rv[c + SA], g.dmv[c],
+                         g.db1[c], g.db1[c + SA], g.db1[c + 2 * SA], g.dc1[c], g.dc1[c + SA], w, dt, F, fpre);
 #pragma unroll
-    for (int comp = 0; comp < 3; ++comp) g.fp[comp][c] = fpre[comp];
-  }
+  for (int comp = 0; comp < 3; ++comp) g.fp[comp][c] = fpre[comp];
 }
 
 // rke's kinetic-energy defect of one component through the vertex pair
@@ -301,7 +300,7 @@ __device__ __forceinline__ void mom_update(const MomArgs<R>& g, int c, const R (
   for (int comp = 0; comp < 3; ++comp) g.vn[comp][c] = dv_div(rvc * g.v[comp][c] * c1 + Fm[comp] - F[comp], den);
 }
 
-template <class R, bool RKE>
+template <class R>
 __global__ void __launch_bounds__(128) k_mom_x(MomArgs<R> g) {
   const int lane = (int)threadIdx.x;                        // blockDim.x == 32: one warp per row
   const int ix = -1 + (int)blockIdx.x * 31 + lane;          // face / vertex x position
@@ -311,14 +310,14 @@ __global__ void __launch_bounds__(128) k_mom_x(MomArgs<R> g) {
   const R dt = (R)g.sc[g.dt_slot];
   const int c = ix + g.sx * iy + g.sxy * iz;
   R F[3] = {R(0), R(0), R(0)};
-  if (ix <= g.nx) mom_flux<R, RKE>(g, c, iy, iz, dt, F);    // faces -1..n
+  if (ix <= g.nx) mom_flux<R>(g, c, iy, iz, dt, F);    // faces -1..n
   R Fm[3];
 #pragma unroll
   for (int comp = 0; comp < 3; ++comp) Fm[comp] = __shfl_up_sync(0xffffffffu, F[comp], 1);
   if (lane >= 1 && ix >= 0 && ix <= g.nx) mom_update(g, c, Fm, F);
 }
 
-template <class R, bool RKE>
+template <class R>
 __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 4 : 8) k_mom_march(MomArgs<R> g) {
   const int t0 = (int)(blockIdx.x * blockDim.x + threadIdx.x);  // x, 0..nx
   const int t1 = (int)(blockIdx.y * blockDim.y + threadIdx.y);  // the third axis, 0..n3
@@ -339,11 +338,9 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 4 : 8) k_mom_march(MomAr
   R va0 = g.va[c], va1 = g.va[c + SA], rvc = g.rv[c], rvn = g.rv[c + SA];
   R dbw0 = g.db1[c], dbw1 = g.db1[c + SA], dbw2 = g.db1[c + 2 * SA], dcw0 = g.dc1[c], dcw1 = g.dc1[c + SA];
   R Fm[3], fpre[3];
-  mom_flux_vals<R, RKE>(area, va0, va1, rvc, rvn, g.dmv[c], dbw0, dbw1, dbw2, dcw0, dcw1, w, dt, Fm, fpre);
-  if constexpr (RKE) {
+  mom_flux_vals<R, true>(area, va0, va1, rvc, rvn, g.dmv[c], dbw0, dbw1, dbw2, dcw0, dcw1, w, dt, Fm, fpre);
 #pragma unroll
-    for (int comp = 0; comp < 3; ++comp) g.fp[comp][c] = fpre[comp];
-  }
+  for (int comp = 0; comp < 3; ++comp) g.fp[comp][c] = fpre[comp];
   // the loads of face c + SA are issued one step ahead (a face's own values
   // and the new far points of the windows), so each step's arithmetic waits
   // on loads issued a step earlier
@@ -386,11 +383,9 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 4 : 8) k_mom_march(MomAr
     dcw0 = dcw1;
     dcw1 = cur.dc;
     R F[3];
-    mom_flux_vals<R, RKE>(area, va0, va1, rvc, rvn, cur.dm, dbw0, dbw1, dbw2, dcw0, dcw1, w, dt, F, fpre);
-    if constexpr (RKE) {
+    mom_flux_vals<R, true>(area, va0, va1, rvc, rvn, cur.dm, dbw0, dbw1, dbw2, dcw0, dcw1, w, dt, F, fpre);
 #pragma unroll
-      for (int comp = 0; comp < 3; ++comp) g.fp[comp][c] = fpre[comp];
-    }
+    for (int comp = 0; comp < 3; ++comp) g.fp[comp][c] = fpre[comp];
     // K9's update at c: fluxes at faces c - e_A and c
     const R c1 = cur.c1, den = dv_of(cur.c2 * cur.r1);
 #pragma unroll
@@ -425,16 +420,12 @@ void remap_sweep(Run<R>& run, int dt_slot, int pass[3], int bmode) {
   R* const vz1 = Ar.vz1.p;
   R* const V1[3] = {vx1, vy1, vz1};
   R* const va = V1[A];
-  R* const cv = Ar.cv.p;
   R* const cv1 = Ar.cv1.p;
   R* const db1 = Ar.db1.p;
   R* const dc1 = Ar.dc1.p;
   const A1<R> dbm[3] = {Ar.dxb, Ar.dyb, Ar.dzb};
   const A1<R> dcm[3] = {Ar.dxc, Ar.dyc, Ar.dzc};
-  const A1<R> dba = dbm[A], dbt1 = dbm[T1], dbt2 = dbm[T2], dct1 = dcm[T1], dct2 = dcm[T2];
-  const A1<R> rdba = Ar.rdb[A], rdbt1 = Ar.rdb[T1], rdbt2 = Ar.rdb[T2];
-  const R pass_t1 = (R)pass[T1], pass_t2 = (R)pass[T2];
-  const double* sc = run.sc;
+  const A1<R> dct1 = dcm[T1], dct2 = dcm[T2];
 
   // ---- K1: B, into the arrays of the Lagrangian step's B0, whose work is done
   // (bx1, by1, bz1 are named fields: the B before the last resistive sub-cycle)
@@ -552,8 +543,7 @@ void remap_sweep(Run<R>& run, int dt_slot, int pass[3], int bmode) {
     gm.sxy = sxy;
     gm.SA = SA;
     gm.S3 = A == 1 ? sxy : sx;
-    const bool rke = run.p.rke != 0;
-    for (int q = 0; q < 3; ++q) gm.fp[q] = rke ? Ar.rke_f[q].p : nullptr;
+    for (int q = 0; q < 3; ++q) gm.fp[q] = Ar.rke_f[q].p;
     if (fused_vm) {
       VMArgs<R> vm;
       vm.m = gm;
@@ -564,22 +554,16 @@ void remap_sweep(Run<R>& run, int dt_slot, int pass[3], int bmode) {
       vm.dm = dm;
       vm_launch<A>(run, vm);
     } else {
-      const int k = run.prof_begin(A == 0 ? "remap_sweep_mom_x" : "remap_sweep_mom_march", 0, rke ? 17 : 14,
+      const int k = run.prof_begin(A == 0 ? "remap_sweep_mom_x" : "remap_sweep_mom_march", 0, 17,
                                    (double)(nx + 1) * (ny + 1) * (nz + 1));
       if (A == 0) {
         dim3 grd((nx + 1 + 30) / 31, (ny + 1 + 3) / 4, nz + 1);
-        if (rke)
-          k_mom_x<R, true><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
-        else
-          k_mom_x<R, false><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
+        k_mom_x<R><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
       } else {
         dim3 grd((nx + 1 + 31) / 32, (gm.n3 + 1 + 3) / 4, 1);
-        gm.chunk = march_chunk(na + 1, grd.x * grd.y, kMomA, resident_blocks<k_mom_march<R, true>>(128));
+        gm.chunk = march_chunk(na + 1, grd.x * grd.y, kMomA, resident_blocks<k_mom_march<R>>(128));
         grd.z = (na + 1 + gm.chunk - 1) / gm.chunk;
-        if (rke)
-          k_mom_march<R, true><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
-        else
-          k_mom_march<R, false><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
+        k_mom_march<R><<<grd, dim3(32, 4, 1), 0, run.s>>>(gm);
       }
       run.prof_end(k);
       ++run.launches;
