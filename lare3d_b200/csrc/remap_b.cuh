@@ -17,11 +17,11 @@
 // Every value is the reference's expression over the same operands in the
 // same order, so the exact build stays bit for bit.
 //
-// At 256^3 a sweep takes 0.28 ms (y, z) and 0.30 ms (x) in FP64 and 0.19 ms in
-// FP32, against 0.70 and 0.44 ms for the three kernels; the floor is its 7
-// words, 0.145 ms in FP64.  Bound by instruction issue (62 % of slots with the
-// 16 warps an SM that the windows' registers allow) and by the halo, 28 % of
-// the tiles' points.  Measured and not kept: planes prefetched into registers
+// At 256^3 a sweep takes 0.29 ms (y, z) and 0.30 ms (x) in FP64 and 0.20 to 0.24
+// ms in FP32, against 0.70 and 0.44 ms for the three kernels; the floor is its 7
+// words, 0.15 ms in FP64.  Bound by instruction issue (57 to 61 % of slots with
+// the 16 warps an SM that the windows' registers allow; about 80 % in FP32) and
+// by the halo, 15 (y, z) to 26 % (x) of the tiles' lanes.  Measured and not kept: planes prefetched into registers
 // instead of the ring (0.50 ms: too little in flight for the DRAM latency), one
 // component a thread on 512-thread blocks (0.37 ms: the barrier and the
 // geometry formed twice), tiles of 4, 12 and 16 rows (0.31, 0.34, 0.31 ms).

@@ -14,10 +14,10 @@
 // components still to come (SWEPT: how many of the two other axes are done;
 // the third sweep's cv2 is cv itself and is not written).
 //
-// At 256^3 a sweep takes 0.32 (y, z) and 0.36 ms (x) in FP64, 0.22 and 0.25 ms
-// in FP32, where the geometry kernel and this one took 0.59 and 0.67, 0.35 and
-// 0.41 ms; its floor is 0.23 ms (11 words, FP64).  Bound by instruction issue
-// and FP64 latency at 16 warps an SM.  With plain loads a step ahead instead of
+// At 256^3 a sweep takes 0.30 to 0.37 (y, z) and 0.40 ms (x) in FP64 with the
+// components still to come, 0.24 ms in FP32, where the geometry kernel and this
+// one took 0.59 and 0.67, 0.35 and 0.41 ms; its floor is 0.23 ms (11 words, FP64).
+// Bound by instruction issue (55 % of slots) and FP64 latency at 16 warps an SM.  With plain loads a step ahead instead of
 // the ring: 0.54 and 0.53 ms (168 registers, waiting on memory).
 //
 // The fluxes of the point below are carried, so neither flux but dm reaches

@@ -9,7 +9,7 @@
 // read these back.  Here the momentum kernel forms them on the way, and the
 // moved widths db1 and dc1 from the face velocity, so no vertex or geometry
 // array reaches memory (11 words per point instead of 9 + 14).  At 256^3 a
-// sweep takes 0.33 ms (y, z) and 0.36 ms (x) in FP64 and 0.25 and 0.24 ms in
+// sweep takes 0.34 ms (y, z) and 0.37 ms (x) in FP64 and 0.26 and 0.25 ms in
 // FP32; reading db1 and dc1 with plain loads it took 0.46 and 0.36, 0.30 and
 // 0.32 ms.  The floor is 0.23 ms (FP64); bound by issue at 16 warps an SM.
 //
